@@ -41,7 +41,9 @@
 // two steps read come from per-warpgroup shared-memory rings that a non-issuing warp fills by
 // cp.async, eight wavelets ahead of use: read from L2 they put two L2 latencies on every
 // wavelet's chain.  Warpgroups take tiles from a per-launch counter, so tiles of different
-// cost (requests of different K) balance across the SMs.  The two standard networks run
+// cost (requests of different K) balance across the SMs; the tiles that would leave most chains
+// idle (a small launch, a large one's last round) are shared by a CTA's five warpgroups, a fifth
+// of the wavelets each (the launcher's rule has the figures).  The two standard networks run
 // kernels specialised on their layer sequence (ShapeOf), every other supported network a
 // generic form that reads the sequence from the plan.  Every wait is bounded by
 // %globaltimer (2 s); on expiry the kernel records kDevWaitTimeout and the warpgroup
@@ -91,12 +93,15 @@ struct TcParams {
   int enc_dims;  // D, multiple of 16, <= 32
   TcJob jobs[kInlineJobs];
   int n_jobs;
-  long long total_tiles;
+  int total_tiles;
   int kahan, clamp;
   float cp_scale;   // FP8: scale of the first layer's operand
   uint32_t* amax;   // calibration: per-layer activation maxima (float bits)
   uint32_t* err;
-  int* tile_ctr;    // the next 128-pixel tile to take (zeroed before the launch)
+  int* tile_ctr;    // tiles taken beyond the warpgroups' first ones (zeroed before the launch);
+                    // null when every warpgroup has at most its first tile
+  int whole_tiles;        // tiles [0, whole_tiles) go to one warpgroup each; for the rest a CTA's
+                          // warpgroups share a tile, one chunk of its wavelets each
   // Shared-memory descriptors of every layer's B tile, its aux block and the output layer's
   // FP16 tile, formed on the host with the weight region at address 0: the kernel adds the
   // region's address (>> 4, no carry out of the 14-bit field below 256 KB) in one step.
@@ -165,6 +170,14 @@ __device__ __forceinline__ bool wg_barrier_and(int g, bool pred) {
       : "r"((uint32_t)pred), "r"(1 + g)
       : "memory");
   return out != 0;
+}
+
+// Named barriers 6..9 order the warpgroups' first tiles: a warpgroup arrives, the next one waits.
+__device__ __forceinline__ void named_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void named_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
 __host__ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
@@ -404,13 +417,24 @@ __device__ __forceinline__ void final_dot32x2(const uint32_t (&v)[32], const flo
   }
 }
 
-// Hash-grid encoding (same arithmetic as the FP32 path), kept as BF16 pairs.
-template <int DMAX>
-__device__ __forceinline__ void hash_encode_bf16(const HashLevels& hl, const float* __restrict__ table,
-                                                 float px, float py, float pz, uint32_t (&enc)[DMAX / 2]) {
+// Levels l0, l0 + step, ... < l1 of the hash-grid encoding of one position per lane (the same
+// arithmetic, in the same order, as the FP32 path), each level's BF16 feature pair handed to
+// put(l, pair).  All 32 lanes take part.
+//
+// The random table reads bound it: the SM serves one 128-byte line per cycle to gathered loads
+// (measured: 27 us per 640-pixel CTA round at 85% of that rate, whether 26 or 148 SMs run).  The
+// two corners of a cell edge along x are table neighbours and mostly share a line, so lanes 2j
+// and 2j + 1 load each other's: one load brings both x corners of the even lane's cell (one per
+// lane), the next both of the odd lane's, and a shuffle hands the foreign halves over.  A load
+// then touches about 17 lines instead of 32: 38.4 -> 29.6 us per 640 pixels x 148 SMs (random
+// positions, 2^19-entry tables); 16- and 32-byte loads that span the neighbour: 33.9 and 35.1 us.
+template <class PUT>
+__device__ __forceinline__ void hash_encode_pairs(const HashLevels& hl, const float* __restrict__ table, float px,
+                                                  float py, float pz, int l0, int l1, int step, const PUT& put) {
   const float p[3] = {fminf(fmaxf(px, 0.f), 1.f), fminf(fmaxf(py, 0.f), 1.f), fminf(fmaxf(pz, 0.f), 1.f)};
-#pragma unroll
-  for (int l = 0; l < DMAX / 2; ++l) {
+  const bool odd = threadIdx.x & 1;
+#pragma unroll 2
+  for (int l = l0; l < l1; l += step) {
     float a0 = 0.f, a1 = 0.f;
     if (l < hl.n_levels) {
       const int N = hl.res[l];
@@ -428,22 +452,31 @@ __device__ __forceinline__ void hash_encode_bf16(const HashLevels& hl, const flo
       const bool dense = (hl.dense_mask >> l) & 1u;
       const uint32_t T = hl.size[l];
       const float2* lvl = reinterpret_cast<const float2*>(table) + hl.offset[l];
+      float2 first[4], second[4];  // of the even lane's cell and of the odd lane's: this lane's x corner
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const uint32_t bx = c & 1, by = (c >> 1) & 1, bz = (c >> 2) & 1;
-        const float wx = bx ? w[0] : __fsub_rn(1.f, w[0]);
-        const float wy = by ? w[1] : __fsub_rn(1.f, w[1]);
-        const float wz = bz ? w[2] : __fsub_rn(1.f, w[2]);
-        const float wc = __fmul_rn(__fmul_rn(wx, wy), wz);
-        const uint32_t x = i0[0] + bx, y = i0[1] + by, z = i0[2] + bz;
-        const uint32_t e = dense ? x + y * N1 + z * N1 * N1
-                                 : ((x ^ (y * 2654435761u) ^ (z * 805459861u)) & (T - 1u));
-        const float2 v = __ldg(lvl + e);
-        a0 = fmaf(wc, v.x, a0);
-        a1 = fmaf(wc, v.y, a1);
+      for (int c = 0; c < 4; ++c) {
+        const uint32_t x = i0[0], y = i0[1] + (c & 1), z = i0[2] + (c >> 1);
+        const uint32_t yz = dense ? y * N1 + z * N1 * N1 : (y * 2654435761u) ^ (z * 805459861u);
+        const uint32_t e0 = dense ? x + yz : (x ^ yz) & (T - 1u);
+        const uint32_t e1 = dense ? x + 1u + yz : ((x + 1u) ^ yz) & (T - 1u);
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, odd ? e0 : e1, 1);
+        first[c] = __ldg(lvl + (odd ? other : e0));
+        second[c] = __ldg(lvl + (odd ? e1 : other));
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float2 mine = odd ? second[c] : first[c], foreign = odd ? first[c] : second[c];
+        const float fx = __shfl_xor_sync(0xffffffffu, foreign.x, 1), fy = __shfl_xor_sync(0xffffffffu, foreign.y, 1);
+        const float wy = (c & 1) ? w[1] : __fsub_rn(1.f, w[1]);
+        const float wz = (c >> 1) ? w[2] : __fsub_rn(1.f, w[2]);
+        const float w0 = __fmul_rn(__fmul_rn(__fsub_rn(1.f, w[0]), wy), wz), w1 = __fmul_rn(__fmul_rn(w[0], wy), wz);
+        a0 = fmaf(w0, odd ? fx : mine.x, a0);
+        a1 = fmaf(w0, odd ? fy : mine.y, a1);
+        a0 = fmaf(w1, odd ? mine.x : fx, a0);
+        a1 = fmaf(w1, odd ? mine.y : fy, a1);
       }
     }
-    enc[l] = pack_bf16(a0, a1);
+    put(l, pack_bf16(a0, a1));
   }
 }
 
@@ -459,7 +492,9 @@ struct EncRow {
       : base(reinterpret_cast<uint4*>(tile_encs) + row * kChunks),
         swz(kChunks == 4 ? (row >> 1) & 3 : (row >> 2) & 1) {}
   __device__ __forceinline__ uint4 get(int c) const { return base[c ^ swz]; }
-  __device__ __forceinline__ void put(int c, uint4 v) const { base[c ^ swz] = v; }
+  __device__ __forceinline__ void put_pair(int l, uint32_t v) const {
+    reinterpret_cast<uint32_t*>(base + ((l >> 2) ^ swz))[l & 3] = v;
+  }
 };
 
 // First-layer operand of wavelet k, hash(p) * E_k -> TMEM A columns.  BF16: one packed
@@ -538,7 +573,35 @@ __device__ __forceinline__ void store_cp_smem(const EncRow<DMAX>& enc, const uin
   else tmem_st8(a_taddr, cp);
 }
 
-__device__ __forceinline__ int find_job(const TcJob* jobs, int n_jobs, long long tile) {
+// Adds a chunk's channel sums s (with their Kahan compensations c: the sum is s - c) to a pixel's
+// running ones at tot, [6][kTile]: three sums, three compensations.  init: tot's first chunk.
+__device__ __forceinline__ void add_chunk(float* tot, bool init, int kahan, float s0, float s1, float s2, float c0,
+                                          float c1, float c2) {
+  const float s[3] = {s0, s1, s2}, c[3] = {c0, c1, c2};
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    float S = s[i], C = c[i];
+    if (!init) {
+      S = tot[i * kTile];
+      C = tot[(3 + i) * kTile];
+      if (kahan) {
+        float y = __fsub_rn(s[i], C), z = __fadd_rn(S, y);
+        C = __fsub_rn(__fsub_rn(z, S), y);
+        S = z;
+        y = __fsub_rn(-c[i], C);
+        z = __fadd_rn(S, y);
+        C = __fsub_rn(__fsub_rn(z, S), y);
+        S = z;
+      } else {
+        S = __fadd_rn(S, s[i]);
+      }
+    }
+    tot[i * kTile] = S;
+    tot[(3 + i) * kTile] = C;
+  }
+}
+
+__device__ __forceinline__ int find_job(const TcJob* jobs, int n_jobs, int tile) {
   int lo = 0, hi = n_jobs - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -608,7 +671,7 @@ __device__ __forceinline__ void issue_steps(uint32_t d_tmem, uint32_t a_tmem, ui
 // made every layer's round trip measurably longer.
 template <int MODE>
 __device__ __forceinline__ void issue_layer(const TcLayer& L, bool with_aux, uint32_t wbase, uint32_t a_tmem,
-                                            uint32_t aux_base, uint32_t d_tmem, uint64_t* bar) {
+                                            uint64_t ad, uint32_t d_tmem, uint64_t* bar) {
   tc_fence_after();
   const uint64_t b0 = smem_desc(wbase + L.b_off, 128u, L.b_sbo);
   const uint32_t id = MODE == kTcFp8 ? idesc_e4m3(L.n) : idesc_bf16(L.n);
@@ -618,7 +681,6 @@ __device__ __forceinline__ void issue_layer(const TcLayer& L, bool with_aux, uin
   else if (steps == 1) issue_steps<MODE, 1>(d_tmem, a_tmem, b0, id);
   else issue_steps<MODE, 3>(d_tmem, a_tmem, b0, id);
   if (with_aux) {
-    const uint64_t ad = smem_desc(aux_base, 128u, 256u);
     const uint64_t bd = smem_desc(wbase + L.aux_off, 128u, 256u);
     mma_ss(d_tmem, ad, bd, idesc_bf16(L.n), 1u);
   }
@@ -650,7 +712,8 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
   uint8_t* wsm = smem;                                                  // weight blob
   uint8_t* aux = smem + weight_region_bytes(p.w_boxes, p.w_box_rows);  // [kNWG][kAuxBytes]
   uint32_t* encs = reinterpret_cast<uint32_t*>(aux + kNWG * kAuxBytes);  // [kNWG][kTile][DMAX/2], swizzled
-  TcBarriers* bars = reinterpret_cast<TcBarriers*>(encs + kNWG * (DMAX / 2) * kTile);
+  float* sums = reinterpret_cast<float*>(encs + kNWG * (DMAX / 2) * kTile);  // [kNWG][6][kTile] sums of chunks
+  TcBarriers* bars = reinterpret_cast<TcBarriers*>(sums + kNWG * 6 * kTile);
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   const int g = warp >> 2;  // warpgroup
@@ -679,8 +742,7 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  // the weights have landed (every thread sees the barrier complete before any MMA reads them)
-  bool ok = wait_bounded(&bars->wload, 0, p.err);
+  bool ok = true;
   const uint32_t tmem = bars->tmem_base;
   const uint32_t wbase = smem_u32(wsm);
   const uint32_t col0 = tmem + (uint32_t)(g * kTileCols);
@@ -716,53 +778,87 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
         issue_fixed<MODE, kS1, false>(p.bdesc[nl] + wb16, aux_desc, 0ull, a_tmem, d_tmem, acc_bar);
       }
     } else {
-      issue_layer<MODE>(p.layers[nl], Sh::aux >= 0 ? Sh::aux == nl : p.layers[nl].aux != 0, wbase, a_tmem, aux_base,
+      issue_layer<MODE>(p.layers[nl], Sh::aux >= 0 ? Sh::aux == nl : p.layers[nl].aux != 0, wbase, a_tmem, aux_desc,
                         d_tmem, acc_bar);
     }
   };
 
   uint32_t ph = 0;
-  // Tiles come from the launch's counter, one atomic per tile and warpgroup, so that tiles of
-  // different cost (jobs of different K or pixel count; the host puts the longest tiles first)
-  // balance across the SMs.  The slot is read after a warpgroup barrier and rewritten only after
-  // the next one (every tile has at least one).
-  if (q == 0 && lane == 0) bars->tile_slot[g] = atomicAdd(p.tile_ctr, 1);
-  ok = wg_barrier_and(g, ok);
-  for (long long t = bars->tile_slot[g]; t < p.total_tiles && ok; t = bars->tile_slot[g]) {
-    // ---- tile set-up: hash encoding, aux operand, first-layer operand of wavelet 0
+  // Which warpgroup does what.  Whole tiles: warpgroup g of CTA b starts with tile g * grid + b
+  // and takes further ones from the launch's counter, so that tiles of different cost (jobs of
+  // different K or pixel count; the host puts the longest tiles first) balance across the SMs.
+  // The counter's value is read after a warpgroup barrier and the slot rewritten only after the
+  // next one (every tile has at least one).  Shared tiles, after them: the CTA's warpgroups work
+  // on one tile, a chunk of its wavelets each (few tiles would leave most chains idle).
+  int t = p.whole_tiles == 0 ? (int)blockIdx.x : g * (int)gridDim.x + (int)blockIdx.x;
+  // The first tiles' hash encodings are staggered: warpgroup g + 1 starts when g has two thirds
+  // of its levels.  Their rate is the SM's anyway, and started together no chain would run until
+  // all five are done; started in turn, the first chain runs after a fifth of the time.
+  if (p.whole_tiles > 0 && g > 0) named_sync(5 + g, 256);
+  if (p.whole_tiles > 0 && g + 1 < kNWG && t >= p.whole_tiles) named_arrive(6 + g, 256);
+  // This warpgroup is done with whole tiles: its first shared tile, after the CTA's others are too.
+  auto leave_whole = [&]() -> int {
+    if (p.whole_tiles == p.total_tiles) return p.total_tiles;
+    ok = __syncthreads_and(ok);
+    return p.whole_tiles + (int)blockIdx.x;
+  };
+  if (p.whole_tiles > 0 && t >= p.whole_tiles) t = leave_whole();
+  while (t < p.total_tiles && ok) {
+    // ---- tile set-up: hash encoding, aux operand, first-layer operand of the first wavelet
     const int jid = find_job(p.jobs, p.n_jobs, t);
     const TcJob& J = p.jobs[jid];
-    const int K = J.K;
+    // The sum over K wavelets is the sum, in order, of the sums of kNWG chunks of ceil(K / kNWG)
+    // wavelets, in every launch: a result's bits do not depend on how the launch was split.
+    auto chunk = [&] { return (J.K + kNWG - 1) / kNWG; };
+    auto shared_tile = [&] { return t >= p.whole_tiles; };
+    auto k_begin = [&] { return shared_tile() ? min(g * chunk(), J.K) : 0; };
+    // this warpgroup's wavelets: [k_begin, k_begin + K)
+    const int K = shared_tile() ? min(chunk(), J.K - k_begin()) : J.K;
     const long long px = J.px_begin + (t - J.tile_begin) * kTile + row;
     const bool valid = px < J.n_px;
-    const EncRow<DMAX> enc_s(encs + g * (DMAX / 2) * kTile, row);  // this pixel's features
-    if (valid) {
-      uint32_t enc[DMAX / 2];
-      const float4* pr = reinterpret_cast<const float4*>(J.packed) + px * 4;
-      const float4 r0 = __ldg(pr), r1 = __ldg(pr + 1), r2 = __ldg(pr + 2), r3 = __ldg(pr + 3);
-      hash_encode_bf16<DMAX>(p.hl, p.hash, r0.x, r0.y, r0.z, enc);
-#pragma unroll
-      for (int c = 0; c < DMAX / 8; ++c)
-        enc_s.put(c, make_uint4(enc[4 * c], enc[4 * c + 1], enc[4 * c + 2], enc[4 * c + 3]));
-      // aux operand: the 13 remapped G-buffer values followed by ones
-      st_shared_v4(aux_row, pack_bf16(r0.w, r1.x), pack_bf16(r1.y, r1.z), pack_bf16(r1.w, r2.x),
-                   pack_bf16(r2.y, r2.z));
-      st_shared_v4(aux_row + 128u, pack_bf16(r2.w, r3.x), pack_bf16(r3.y, r3.z), pack_bf16(r3.w, 1.f),
-                   pack_bf16(1.f, 1.f));
-    } else {
-#pragma unroll
-      for (int c = 0; c < DMAX / 8; ++c) enc_s.put(c, make_uint4(0u, 0u, 0u, 0u));
-      st_shared_v4(aux_row, 0, 0, 0, 0);
-      st_shared_v4(aux_row + 128u, 0, 0, 0, 0);
+    // this pixel's features (those of a shared tile: in warpgroup 0's region)
+    const EncRow<DMAX> enc_s(encs + (shared_tile() ? 0 : g) * (DMAX / 2) * kTile, row);
+    {
+      const float4* pr = reinterpret_cast<const float4*>(J.packed) + (valid ? px : J.n_px - 1) * 4;
+      const float4 r0 = __ldg(pr);
+      auto put = [&](int l, uint32_t v) { enc_s.put_pair(l, valid ? v : 0u); };
+      if (shared_tile()) {
+        hash_encode_pairs(p.hl, p.hash, r0.x, r0.y, r0.z, g, DMAX / 2, kNWG, put);
+      } else {
+        constexpr int kPart = DMAX / 3;
+        hash_encode_pairs(p.hl, p.hash, r0.x, r0.y, r0.z, 0, kPart, 1, put);
+        if (g + 1 < kNWG && t < kNWG * (int)gridDim.x) named_arrive(6 + g, 256);  // the first tile
+        hash_encode_pairs(p.hl, p.hash, r0.x, r0.y, r0.z, kPart, DMAX / 2, 1, put);
+      }
+      if (valid) {
+        // aux operand: the 13 remapped G-buffer values followed by ones
+        const float4 r1 = __ldg(pr + 1), r2 = __ldg(pr + 2), r3 = __ldg(pr + 3);
+        st_shared_v4(aux_row, pack_bf16(r0.w, r1.x), pack_bf16(r1.y, r1.z), pack_bf16(r1.w, r2.x),
+                     pack_bf16(r2.y, r2.z));
+        st_shared_v4(aux_row + 128u, pack_bf16(r2.w, r3.x), pack_bf16(r3.y, r3.z), pack_bf16(r3.w, 1.f),
+                     pack_bf16(1.f, 1.f));
+      } else {
+        st_shared_v4(aux_row, 0, 0, 0, 0);
+        st_shared_v4(aux_row + 128u, 0, 0, 0, 0);
+      }
     }
-    store_cp<DMAX, MODE>(enc_s, J.emb_k, J.emb_h, a_taddr, p.cp_scale, p.amax);
-    tmem_wait_st();
+    // the weights have landed (every thread sees the barrier complete before any MMA reads them)
+    ok = wait_bounded(&bars->wload, 0, p.err) && ok;
+    if (shared_tile()) ok = __syncthreads_and(ok);  // the tile's features are complete
     float s0 = 0.f, s1 = 0.f, s2 = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f;
-    // hand the first layer to the tensor core
-    tc_fence_before();
-    fence_proxy_async_smem();
-    ok = wg_barrier_and(g, ok);
-    if (ok && q == lead && elect_one()) issue_next(0);
+    int flush_at = shared_tile() ? 0 : chunk();  // the wavelet that the next chunk starts with (0: never)
+    if (K > 0) {
+      const int kb = k_begin();
+      store_cp<DMAX, MODE>(enc_s, J.emb_k + (size_t)kb * p.enc_dims, J.emb_h + (size_t)kb * (p.enc_dims / 2), a_taddr,
+                           p.cp_scale, p.amax);
+      tmem_wait_st();
+      // hand the first layer to the tensor core
+      tc_fence_before();
+      fence_proxy_async_smem();
+      ok = wg_barrier_and(g, ok);
+      if (ok && q == lead && elect_one()) issue_next(0);
+    }
+    float* my_sums = sums + g * 6 * kTile + row;
     // T_k -> clamped Kahan sums, then the next wavelet's first-layer operand
     auto finish_wavelet = [&](int k, float t0, float t1, float t2) {
       float L0, L1, L2;
@@ -770,7 +866,7 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
         const float4 Lk = bars->l_ring[g][k % kRing];
         L0 = Lk.x; L1 = Lk.y; L2 = Lk.z;
       } else {
-        const float* Lk = J.strength + (size_t)k * 3;
+        const float* Lk = J.strength + (size_t)(k_begin() + k) * 3;
         L0 = __ldg(Lk + 0); L1 = __ldg(Lk + 1); L2 = __ldg(Lk + 2);
       }
       float u0 = __fmul_rn(L0, t0);
@@ -785,9 +881,15 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
       } else {
         s0 = __fadd_rn(s0, u0); s1 = __fadd_rn(s1, u1); s2 = __fadd_rn(s2, u2);
       }
+      if (k + 1 == flush_at) {  // the chunk's sums join the tile's
+        add_chunk(my_sums, flush_at == chunk(), p.kahan, s0, s1, s2, c0, c1, c2);
+        s0 = s1 = s2 = c0 = c1 = c2 = 0.f;
+        flush_at += chunk();
+      }
       if (!OUT_TC && k + 1 < K) {  // OUT_TC: written while the output layer's MMA runs
-        store_cp<DMAX, MODE>(enc_s, J.emb_k + (size_t)(k + 1) * p.enc_dims,
-                             J.emb_h + (size_t)(k + 1) * (p.enc_dims / 2), a_taddr, p.cp_scale, p.amax);
+        const int kn = k_begin() + k + 1;
+        store_cp<DMAX, MODE>(enc_s, J.emb_k + (size_t)kn * p.enc_dims, J.emb_h + (size_t)kn * (p.enc_dims / 2),
+                             a_taddr, p.cp_scale, p.amax);
         tmem_wait_st();
       }
     };
@@ -892,13 +994,13 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
           // E_k+1..k+8 and L_k..k+7 into the rings, by a warp that would otherwise only wait
           // for this layer's MMAs; waited for before this wavelet's last hidden-layer barrier
           constexpr int C = DMAX / 8;
-          const int j = lane / C;
+          const int j = lane / C, kb = k_begin();
           if (j < kBatch && k + 1 + j < K)
             cp_async16(smem_u32(&bars->e_ring[g][(k + 1 + j) % kRing][lane % C]),
-                       J.emb_h + (size_t)(k + 1 + j) * (p.enc_dims / 2) + (lane % C) * 4);
+                       J.emb_h + (size_t)(kb + k + 1 + j) * (p.enc_dims / 2) + (lane % C) * 4);
           if (lane < 3 * kBatch && k + lane / 3 < K)
             cp_async4(smem_u32(reinterpret_cast<float*>(&bars->l_ring[g][(k + lane / 3) % kRing]) + lane % 3),
-                      J.strength + (size_t)k * 3 + lane);
+                      J.strength + (size_t)(kb + k) * 3 + lane);
           cp_async_commit();
         }
         // T_k's clamped Kahan update waits one more step: under the next wavelet's second layer,
@@ -912,16 +1014,40 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
         }
       }
     }
-    if (valid && ok) {
-      const float4 ind = J.flag[px] ? make_float4(s0, s1, s2, 1.f) : make_float4(0.f, 0.f, 0.f, 1.f);
-      const float4 dl = __ldg(reinterpret_cast<const float4*>(J.direct) + px);
-      reinterpret_cast<float4*>(J.indirect)[px] = ind;
-      reinterpret_cast<float4*>(J.with_direct)[px] =
-          make_float4(__fadd_rn(ind.x, dl.x), __fadd_rn(ind.y, dl.y), __fadd_rn(ind.z, dl.z), 1.f);
+    if (shared_tile()) {
+      // the chunks' sums meet in warpgroup 0, in order
+      add_chunk(my_sums, true, p.kahan, s0, s1, s2, c0, c1, c2);
+      ok = __syncthreads_and(ok);
+      if (g == 0)
+        for (int j = 1; j * chunk() < J.K; ++j) {
+          const float* o = my_sums + j * 6 * kTile;
+          add_chunk(my_sums, false, p.kahan, o[0], o[kTile], o[2 * kTile], o[3 * kTile], o[4 * kTile], o[5 * kTile]);
+        }
+    } else if (flush_at - chunk() < K) {
+      add_chunk(my_sums, flush_at == chunk(), p.kahan, s0, s1, s2, c0, c1, c2);  // the last, shorter chunk
     }
-    // every thread of the warpgroup agrees on the outcome (and sees the next tile) before it
-    if (q == 0 && lane == 0) bars->tile_slot[g] = atomicAdd(p.tile_ctr, 1);
-    ok = wg_barrier_and(g, ok);
+    if (ok && (!shared_tile() || g == 0)) {
+      const long long px = J.px_begin + (t - J.tile_begin) * kTile + row;
+      if (px < J.n_px) {
+        const float4 ind = J.flag[px] ? make_float4(my_sums[0], my_sums[kTile], my_sums[2 * kTile], 1.f)
+                                      : make_float4(0.f, 0.f, 0.f, 1.f);
+        const float4 dl = __ldg(reinterpret_cast<const float4*>(J.direct) + px);
+        reinterpret_cast<float4*>(J.indirect)[px] = ind;
+        reinterpret_cast<float4*>(J.with_direct)[px] =
+            make_float4(__fadd_rn(ind.x, dl.x), __fadd_rn(ind.y, dl.y), __fadd_rn(ind.z, dl.z), 1.f);
+      }
+    }
+    // every thread of the warpgroup (of the CTA, after a shared tile) agrees on the outcome and
+    // sees the next tile before it
+    if (shared_tile()) {
+      ok = __syncthreads_and(ok);
+      t += (int)gridDim.x;
+    } else {
+      if (p.tile_ctr && q == 0 && lane == 0) bars->tile_slot[g] = atomicAdd(p.tile_ctr, 1);
+      ok = wg_barrier_and(g, ok);
+      t = p.tile_ctr ? kNWG * (int)gridDim.x + bars->tile_slot[g] : p.whole_tiles;
+      if (t >= p.whole_tiles || !ok) t = leave_whole();
+    }
   }
   if (OUT_TC && q == fetcher) cp_async_wait_all();  // no ring copy outlives the CTA (a timed-out exit)
   // every MMA this warpgroup issued has completed before TMEM is released
@@ -1255,7 +1381,8 @@ void weight_boxes(uint32_t blob_bytes, uint32_t* rows, uint32_t* boxes, uint32_t
 size_t smem_for_blob(const NetDims& d, uint32_t blob_bytes) {
   uint32_t rows, boxes, box_rows;
   weight_boxes(blob_bytes, &rows, &boxes, &box_rows);
-  return weight_region_bytes(boxes, box_rows) + (size_t)kNWG * kAuxBytes + enc_smem_bytes(d) + sizeof(TcBarriers);
+  return weight_region_bytes(boxes, box_rows) + (size_t)kNWG * kAuxBytes + enc_smem_bytes(d) +
+         (size_t)kNWG * 6 * kTile * sizeof(float) + sizeof(TcBarriers);
 }
 
 size_t relight_tc_smem_bytes(const NetDims& d) { return smem_for_blob(d, (uint32_t)tc_weight_bytes(d)); }
@@ -1347,19 +1474,34 @@ void launch_relight_tc(const NetDims& d, const HashLevels& hl, const float* hash
     tiles += (p.jobs[i].n_px - p.jobs[i].px_begin + kTile - 1) / kTile;
   }
   if (tiles == 0) return;
-  p.total_tiles = tiles;
+  if (tiles > INT32_MAX / 2) fail(NWPRT_INVALID_ARG, "tensor-core relight: too many tiles in one launch");
+  p.total_tiles = (int)tiles;
   int dev = 0, sms = 0, max_smem = 0;
   NWPRT_CUDA(cudaGetDevice(&dev));
   NWPRT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   NWPRT_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const size_t smem = smem_for_blob(d, P.blob_bytes);
   if (smem > (size_t)max_smem) fail(NWPRT_UNSUPPORTED, "tensor-core relight: shared memory budget exceeded");
-  const long long groups = (tiles + kNWG - 1) / kNWG;
-  const int grid = (int)(groups < sms ? groups : sms);
-  p.tile_ctr = tile_ctr;
+  const int grid = (int)(tiles < sms ? tiles : sms);
+  // Which tiles are shared by a CTA's warpgroups.  In a round (one wavelet per chain) an SM's m
+  // whole tiles take 2.26 us at m = 1, 2.72 at m = 4 and 2.95 at m = 5 (six 64-wide layers), so
+  // the last, partial round of whole tiles costs almost a full one; n shared tiles per SM cost
+  // 0.6 n of such a round, plus ~10 us each for a hash encoding that nothing overlaps.  So when a
+  // partial round leaves n <= 4 tiles per SM, they are shared, if K is large enough to pay for
+  // the encodings (measured at 256 x 256, n = 4: K = 16 87.7 shared and 85.6 us whole, K = 64 203
+  // and 220; at 128 x 128, n = 1: K = 64 229 us before, 162 spread over the SMs, 57 shared).  A
+  // launch of several rounds does it only when all tiles cost the same: tiles of different K
+  // balance through the counter, and leave no common point at which a CTA could change over.
+  const int k_min = p.jobs[n_jobs - 1].K, k_max = p.jobs[0].K;
+  const long long full = tiles - tiles % ((long long)kNWG * sms), rest = tiles - full;
+  const long long per_sm = (rest + sms - 1) / sms;
+  const bool share = per_sm <= 4 && k_min >= 12 * (per_sm - 1) && (full == 0 || k_min == k_max);
+  p.whole_tiles = (int)(share ? full : tiles);
+  const bool counted = p.whole_tiles > (long long)kNWG * grid;
+  p.tile_ctr = counted ? tile_ctr : nullptr;
   auto go = [&](auto kern) {
     NWPRT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    NWPRT_CUDA(cudaMemsetAsync(tile_ctr, 0, sizeof(int), st));
+    if (counted) NWPRT_CUDA(cudaMemsetAsync(tile_ctr, 0, sizeof(int), st));
     kern<<<grid, kThreads, smem, st>>>(p);
   };
   const int shape = shape_of(P, d);

@@ -1,0 +1,50 @@
+"""GPU tests of how a tensor-core launch splits its work: whole tiles (one warpgroup each) and
+tiles shared by a CTA's five warpgroups (a chunk of the wavelets each).
+
+The launcher picks the split from the number of 128-pixel tiles, so the same pixels take
+different paths alone, in a small launch and in a large one.  Every path forms the sum over the
+wavelets from the same chunks in the same order: the bits have to be equal."""
+import numpy as np
+import pytest
+
+from neural_wavelet_prt_demo_b200 import netconfig
+from oracle import oracle as O
+from tests.helpers import make_case, psnr
+
+pytestmark = pytest.mark.gpu
+
+PSNR_MIN = 45.0
+
+
+@pytest.mark.parametrize("cfg,K,kahan", [("small", 1, True), ("small", 4, True), ("small", 5, False),
+                                         ("small", 6, True), ("small", 40, True), ("large", 13, True),
+                                         ("large", 40, False)])
+def test_shared_and_whole_tiles_give_the_same_bits(cuda, cfg, K, kahan):
+    from neural_wavelet_prt_demo_b200 import engine as eng
+    # 774 tiles: on 148 SMs, 740 whole ones and a shared rest
+    case = make_case(netconfig.CONFIG_SMALL if cfg == "small" else netconfig.CONFIG_LARGE, 1021, 97, K, seed=K,
+                     hash_scale=0.5, flag_prob=0.9)
+    n = 1021 * 97
+    e = eng.RenderEngine(case.cfg)
+    e.loadWeights(case.weights)
+    env = e.addEnvironmentMap(eng.EnvironmentMap(top_coefficients=case.idx, top_strength=case.strength))
+    fr = eng.FullFrame.from_gbuffer(case.gbuf)
+    e.setFrame(0, fr)
+    e.TCNNPass_p1(0)
+    rc = eng.RenderConfig(precision="bf16", kahan=kahan)
+    e.TCNNPass_p2(env, 0, rc)
+    e.TCNNSync()
+    whole = fr.fbPredictedIndirect.cpu().numpy(), fr.fbPredictedIndirectWithDirect.cpu().numpy()
+    r64 = O.relight_f64(case.bound, case.idx, case.strength)
+    assert psnr(whole[0][:, :3], r64) >= PSNR_MIN
+    # pieces of 1 px to several tiles per SM: shared tiles only (or, at small K, whole ones);
+    # every piece starts its tiles at its own first pixel, so rows change lanes and warps too
+    cuts = [0, 1, 130, 130 + 148 * 128, 130 + 148 * 128 + 149 * 128, n - 127, n]
+    fr.fbPredictedIndirect.fill_(float("nan"))
+    fr.fbPredictedIndirectWithDirect.fill_(float("nan"))
+    for b, end in zip(cuts[:-1], cuts[1:]):
+        e.relightRanges([(env, 0, fr.fbPredictedIndirect, fr.fbPredictedIndirectWithDirect, b, end)], rc)
+    e.TCNNSync()
+    for got, ref in zip((fr.fbPredictedIndirect, fr.fbPredictedIndirectWithDirect), whole):
+        assert np.array_equal(got.cpu().numpy().view(np.uint32), ref.view(np.uint32))
+    e.close()
