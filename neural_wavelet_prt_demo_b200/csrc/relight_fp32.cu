@@ -1,18 +1,25 @@
 // Fused plain-FP32 relight kernel: the drop-in path.
 //
-// One thread owns one pixel for the whole pass.  It encodes the pixel's position with
-// the multiresolution hash grid once, then for each of the env's K wavelets runs
+// A warp owns 32 (or 16) pixels for the whole pass.  Each lane encodes its pixel's position with
+// the multiresolution hash grid once; then for each of the env's K wavelets the warp runs
 //   cp = enc * E_k                         (ptwise_mlt, utils_kernels.h:110-127)
 //   out_prd MLP -> [out_prd || aux] -> cmp_net MLP -> T_k (RGB)  (prt_network.h:73-154)
-//   sum += max(L_k * T_k, 0)               (computeResponse, utils_kernels.h:84-91)
-// keeping T_k in registers: the N x K transport matrix and the K-fold replicated input
-// of the reference never exist.  Every dot product accumulates fmaf(W[j][i], x_i, .) from
-// 0 in ascending i -- the order of the FP32 oracle (oracle/nwprt_oracle.c: dense_f32) --
-// and the K-sum is Kahan-compensated by default.
+// and each lane sums += max(L_k * T_k, 0) of its pixel (computeResponse, utils_kernels.h:84-91),
+// T_k staying in registers: the N x K transport matrix and the K-fold replicated input of the
+// reference never exist.  Every dot product accumulates fmaf(W[j][i], x_i, .) from 0 in ascending
+// i -- the order of the FP32 oracle (oracle/nwprt_oracle.c: dense_f32) -- and the K-sum is
+// Kahan-compensated by default.
 //
-// Layout: all layer weights live in shared memory transposed to [in][out4] so that each
-// input element meets a warp-uniform float4 row (broadcast reads); each thread keeps its
-// activation vector in a private shared-memory column (conflict-free, stride = block size).
+// Bound by the FP32 pipe (fma.rn.f32x2 at 2.2 issue cycles of 2.0 ideal in a register-only loop)
+// and by what surrounds it.  Layout: all layer weights live in shared memory transposed to
+// [in][out], the activations beside them as [row][pixel].  A layer is a small matrix product per
+// warp: a thread holds 16 pixels x 4 outputs (packed pixel pairs) in registers, so a row costs it
+// five 16-byte shared loads for 32 packed FMAs.  One thread per pixel, as this kernel had it,
+// costs 17 loads for the same 32 (the weights are not reused): shared-memory reads bounded it.
+// The warp's rows are its own, so layers need no block barrier.  The rows of a layer are unrolled
+// by 32, the period of the swizzle, which leaves no address arithmetic in the loop.
+// 1080p network, 611 x 407, K = 64: 28.2 -> 16.7 ms (59% of the FP32 pipe's peak; 55.7 kFLOP per
+// evaluation); 128 x 128 network, 128 x 128, K = 64: 610 -> 453 us.
 #include <cmath>
 
 #include "nwprt_internal.cuh"
@@ -40,10 +47,10 @@ struct Fp32Params {
   int clamp, kahan;
 };
 
-// Hash-grid encoding of one position (oracle/nwprt_oracle.c: orc_hash_encode_f32).
-__device__ __forceinline__ void hash_encode(const HashLevels& hl, const float* __restrict__ table,
-                                            float px, float py, float pz, float* act, int stride,
-                                            int row0) {
+// Hash-grid encoding of one position (oracle/nwprt_oracle.c: orc_hash_encode_f32); feature i to put(i, v).
+template <class PUT>
+__device__ __forceinline__ void hash_encode(const HashLevels& hl, const float* __restrict__ table, float px, float py,
+                                            float pz, const PUT& put) {
   const float p[3] = {fminf(fmaxf(px, 0.f), 1.f), fminf(fmaxf(py, 0.f), 1.f),
                       fminf(fmaxf(pz, 0.f), 1.f)};
   const int F = hl.n_features;
@@ -83,7 +90,7 @@ __device__ __forceinline__ void hash_encode(const HashLevels& hl, const float* _
         for (int f = 0; f < F; ++f) acc[f] = fmaf(wc, __ldg(th + f), acc[f]);
       }
     }
-    for (int f = 0; f < F; ++f) act[(row0 + l * F + f) * stride] = acc[f];
+    for (int f = 0; f < F; ++f) put(l * F + f, acc[f]);
   }
 }
 
@@ -102,252 +109,220 @@ __device__ __forceinline__ void f2_fma(unsigned long long& acc, unsigned long lo
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
-// y = act(W x) over one thread's activation column.
-// MODE 0: x_i = act row i.  MODE 1: x_i = act row (ENC + i) * e[i] (the CP product).
-// MODE 2: x_i = act row i for i < OPO, else act row (AUX + i - OPO) (the [out_prd || aux] concat).
-template <int IN, int OUT, bool RELU, int MODE, int NT, int ENC, int AUX, int OPO>
-__device__ __forceinline__ void dense(const float* __restrict__ Wt, float* act,
-                                      const float* __restrict__ e, float* outv) {
-  constexpr int O4 = r4(OUT) / 4;
-  unsigned long long acc2[O4 * 2];  // output pairs (2j, 2j + 1)
-#pragma unroll
-  for (int j = 0; j < O4 * 2; ++j) acc2[j] = 0ull;
-#pragma unroll 4
-  for (int i = 0; i < IN; ++i) {
-    float xi;
-    if (MODE == 0) xi = act[i * NT];
-    else if (MODE == 1) xi = __fmul_rn(act[(ENC + i) * NT], e[i]);
-    else xi = (i < OPO) ? act[i * NT] : act[(AUX + i - OPO) * NT];
-    const unsigned long long x2 = f2_pack(xi, xi);
-    const float4* w4 = reinterpret_cast<const float4*>(Wt + i * O4 * 4);
-#pragma unroll
-    for (int j = 0; j < O4; ++j) {
-      const float4 w = w4[j];
-      f2_fma(acc2[2 * j], f2_pack(w.x, w.y), x2);
-      f2_fma(acc2[2 * j + 1], f2_pack(w.z, w.w), x2);
-    }
-  }
-  float acc[O4 * 4];
-#pragma unroll
-  for (int j = 0; j < O4 * 2; ++j) f2_unpack(acc2[j], acc[2 * j], acc[2 * j + 1]);
-#pragma unroll
-  for (int j = 0; j < OUT; ++j) {
-    const float v = RELU ? fmaxf(acc[j], 0.f) : acc[j];
-    if (outv) outv[j] = v;
-    else act[j * NT] = v;
-  }
-}
-
-// Compile-time network shape: D hash features, out_prd with OPH hidden layers of width W and
-// OPO outputs, cmp_net with CNH hidden layers of width W, AUXW aux inputs, NT threads.
-template <int D, int OPH, int OPO, int CNH, int W, int AUXW, int NT>
-struct Net {
-  static constexpr int kActRows = (W > OPO ? W : OPO);
-  static constexpr int kEnc = kActRows;
-  static constexpr int kAux = kActRows + D;
-  static constexpr int kRows = kAux + AUXW;
-  static constexpr int kCnIn = OPO + AUXW;
-
-  static constexpr int weight_floats() {
-    int f = 0;
-    if (OPH == 0) f += D * r4(OPO);
-    else f += D * r4(W) + (OPH - 1) * W * r4(W) + W * r4(OPO);
-    if (CNH == 0) f += kCnIn * r4(3);
-    else f += kCnIn * r4(W) + (CNH - 1) * W * r4(W) + W * r4(3);
-    return f;
-  }
-
-  __device__ static void eval(const float* sW, float* act, const float* e, float* T) {
-    const float* w = sW;
-    if constexpr (OPH == 0) {
-      dense<D, OPO, false, 1, NT, kEnc, kAux, OPO>(w, act, e, nullptr);
-      w += D * r4(OPO);
-    } else {
-      dense<D, W, true, 1, NT, kEnc, kAux, OPO>(w, act, e, nullptr);
-      w += D * r4(W);
-#pragma unroll 1
-      for (int l = 1; l < OPH; ++l) {
-        dense<W, W, true, 0, NT, kEnc, kAux, OPO>(w, act, nullptr, nullptr);
-        w += W * r4(W);
-      }
-      dense<W, OPO, false, 0, NT, kEnc, kAux, OPO>(w, act, nullptr, nullptr);
-      w += W * r4(OPO);
-    }
-    if constexpr (CNH == 0) {
-      dense<kCnIn, 3, false, 2, NT, kEnc, kAux, OPO>(w, act, nullptr, T);
-    } else {
-      dense<kCnIn, W, true, 2, NT, kEnc, kAux, OPO>(w, act, nullptr, nullptr);
-      w += kCnIn * r4(W);
-#pragma unroll 1
-      for (int l = 1; l < CNH; ++l) {
-        dense<W, W, true, 0, NT, kEnc, kAux, OPO>(w, act, nullptr, nullptr);
-        w += W * r4(W);
-      }
-      dense<W, 3, false, 0, NT, kEnc, kAux, OPO>(w, act, nullptr, T);
-    }
-  }
-
-  static size_t smem_bytes(int w_floats) {
-    return sizeof(float) * ((size_t)w_floats + kMaxKChunk * D + kMaxKChunk * 4 + (size_t)kRows * NT);
-  }
+// ---- the network: its layer sequence, read at run time.  Output widths up to kMaxOut.
+constexpr int kMaxOut = 64;
+constexpr int kMaxNetLayers = 2 * kMaxLayers;
+struct NetLayer {
+  int in, out, relu, mode;  // 0: the activation rows; 1: the CP product; 2: [out_prd || aux]
+  int w_off;                // float offset of the [in][w_stride] block
 };
-
-template <class NET, int D, int AUXW, int NT>
-__global__ void __launch_bounds__(NT, 1) relight_fp32_kernel(Fp32Params p) {
-  extern __shared__ __align__(16) float sm[];
-  float* sW = sm;
-  float* sE = sW + p.w_floats;
-  float* sL = sE + kMaxKChunk * D;
-  float* sAct = sL + kMaxKChunk * 4;
-  const int tid = threadIdx.x;
-  for (int i = tid * 4; i < p.w_floats; i += NT * 4)
-    *reinterpret_cast<float4*>(sW + i) = __ldg(reinterpret_cast<const float4*>(p.w + i));
-  const int64_t px = p.px_begin + (int64_t)blockIdx.x * NT + tid;
-  const bool valid = px < p.n_px;
-  const bool active = valid && p.flag[px] != 0;
-  float* act = sAct + tid;
-  if (valid) {
-    const float4* row = reinterpret_cast<const float4*>(p.packed) + px * 4;
-    const float4 r0 = row[0], r1 = row[1], r2 = row[2], r3 = row[3];
-    if (active) hash_encode(p.hl, p.hash, r0.x, r0.y, r0.z, act, NT, NET::kEnc);
-    const float aux13[13] = {r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z, r2.w, r3.x, r3.y, r3.z, r3.w};
-#pragma unroll
-    for (int i = 0; i < AUXW; ++i) act[(NET::kAux + i) * NT] = i < 13 ? aux13[i] : 1.0f;
-  }
-  float s[3] = {0.f, 0.f, 0.f}, comp[3] = {0.f, 0.f, 0.f};
-  for (int k0 = 0; k0 < p.K; k0 += kMaxKChunk) {
-    const int kc = min(kMaxKChunk, p.K - k0);
-    __syncthreads();
-    for (int i = tid; i < kc * D; i += NT) sE[i] = p.emb_k[(size_t)k0 * D + i];
-    for (int i = tid; i < kc * 3; i += NT) sL[(i / 3) * 4 + i % 3] = p.strength[(size_t)k0 * 3 + i];
-    __syncthreads();
-    if (!active) continue;
-    for (int kk = 0; kk < kc; ++kk) {
-      float T[3];
-      NET::eval(sW, act, sE + kk * D, T);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        float term = __fmul_rn(sL[kk * 4 + c], T[c]);
-        if (p.clamp) term = fmaxf(term, 0.0f);
-        if (p.kahan) {
-          const float y = __fsub_rn(term, comp[c]);
-          const float t = __fadd_rn(s[c], y);
-          comp[c] = __fsub_rn(__fsub_rn(t, s[c]), y);
-          s[c] = t;
-        } else {
-          s[c] = __fadd_rn(s[c], term);
-        }
-      }
-    }
-  }
-  if (valid) {
-    const float4 dl = reinterpret_cast<const float4*>(p.direct)[px];
-    reinterpret_cast<float4*>(p.indirect)[px] = make_float4(s[0], s[1], s[2], 1.f);
-    reinterpret_cast<float4*>(p.with_direct)[px] =
-        make_float4(__fadd_rn(s[0], dl.x), __fadd_rn(s[1], dl.y), __fadd_rn(s[2], dl.z), 1.f);
-  }
-}
-
-// ---- any other supported network: the same arithmetic with the layer sequence read at run
-// time.  Every dot product still accumulates fmaf(W[j][i], x_i, .) from 0 in ascending i, so
-// results are the same bits as the oracle's.  Output widths up to kGenMaxOut.
-constexpr int kGenMaxOut = 64;
-constexpr int kGenMaxLayers = 2 * kMaxLayers;
-struct GenLayer {
-  int in, out, relu, mode;  // mode as in dense(): 0 plain, 1 CP product, 2 [out_prd || aux]
-  int w_off;                // float offset of the [in][round4(out)] block
-};
-struct GenNet {
-  GenLayer l[kGenMaxLayers];
+struct NetSeq {
+  NetLayer l[kMaxNetLayers];
   int n = 0;
+  // rows of the activation array: hidden activations (and the CP product) from 0, aux values from
+  // aux (a multiple of 32), hash features from enc
   int enc = 0, aux = 0, rows = 0, opo = 0, d = 0, auxw = 0;
 };
 
+// Activations of a block's NT pixels, [row][NT] in shared memory.  Within each 128-byte line of
+// 32 pixels the eight 16-byte chunks are XOR-swizzled by row / 4, so that neither the tile reads
+// (one row, a few pixel groups) nor the tile writes (output groups of four rows, one pixel group)
+// meet a bank conflict.  px: pixel within the line.
 template <int NT>
-__device__ __forceinline__ void dense_rt(const GenLayer& L, const GenNet& g, const float* __restrict__ Wt,
-                                         float* act, const float* __restrict__ e, float* outv) {
-  unsigned long long acc2[kGenMaxOut / 2];  // output pairs (2j, 2j + 1)
-#pragma unroll
-  for (int j = 0; j < kGenMaxOut / 2; ++j) acc2[j] = 0ull;
-  const int o4 = (L.out + 3) / 4;
-  for (int i = 0; i < L.in; ++i) {
-    float xi;
-    if (L.mode == 0) xi = act[i * NT];
-    else if (L.mode == 1) xi = __fmul_rn(act[(g.enc + i) * NT], e[i]);
-    else xi = (i < g.opo) ? act[i * NT] : act[(g.aux + i - g.opo) * NT];
-    const unsigned long long x2 = f2_pack(xi, xi);
-    const float4* w4 = reinterpret_cast<const float4*>(Wt + (size_t)i * o4 * 4);
-#pragma unroll
-    for (int j = 0; j < kGenMaxOut / 4; ++j) {
-      if (j < o4) {
-        const float4 w = w4[j];
-        f2_fma(acc2[2 * j], f2_pack(w.x, w.y), x2);
-        f2_fma(acc2[2 * j + 1], f2_pack(w.z, w.w), x2);
-      }
-    }
-  }
-  float acc[kGenMaxOut];
-#pragma unroll
-  for (int j = 0; j < kGenMaxOut / 2; ++j) f2_unpack(acc2[j], acc[2 * j], acc[2 * j + 1]);
-#pragma unroll
-  for (int j = 0; j < kGenMaxOut; ++j) {
-    if (j < L.out) {
-      const float v = L.relu ? fmaxf(acc[j], 0.f) : acc[j];
-      if (outv) outv[j] = v;
-      else act[j * NT] = v;
-    }
-  }
+__device__ __forceinline__ int act_at(int row, int px) {
+  return row * NT + ((((px >> 2) ^ (row >> 2)) & 7) << 2) + (px & 3);
 }
 
+// acc += W[:, i] x_i for rows row0 .. row0 + n of the activations, in ascending order (row0: a
+// multiple of 32).  A thread holds PX pixels (from px0 of its line; pixel pairs packed) x 4
+// outputs.  w: the first weight row at the thread's outputs, rows WS floats apart.
+template <int PX, int WS, int NT>
+__device__ __forceinline__ void mm_rows(unsigned long long (&acc)[4][PX / 2], const float* __restrict__ w,
+                                        const float* act, int row0, int n, int px0) {
+  constexpr int C = PX / 4;  // 16-byte chunks of a thread's pixels in a row
+  auto step = [&](const float* wr, const float* xr, int swz) {
+    unsigned long long xp[PX / 2];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      // (px0 / 4 + c) ^ swz, px0 / 4 being a multiple of C
+      const float4 v = *reinterpret_cast<const float4*>(xr + (((px0 >> 2) ^ (swz & ~(C - 1))) << 2) +
+                                                        ((c ^ (swz & (C - 1))) << 2));
+      xp[2 * c] = f2_pack(v.x, v.y);
+      xp[2 * c + 1] = f2_pack(v.z, v.w);
+    }
+    const float4 v = *reinterpret_cast<const float4*>(wr);
+    const unsigned long long wd[4] = {f2_pack(v.x, v.x), f2_pack(v.y, v.y), f2_pack(v.z, v.z), f2_pack(v.w, v.w)};
+#pragma unroll
+    for (int o = 0; o < 4; ++o)
+#pragma unroll
+      for (int c = 0; c < PX / 2; ++c) f2_fma(acc[o][c], wd[o], xp[c]);
+  };
+  const float* x = act + row0 * NT;
+#pragma unroll 1
+  for (; n >= 32; n -= 32, x += 32 * NT, w += 32 * WS) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) step(w + i * WS, x + i * NT, i >> 2);
+  }
+  int i = 0;
+#pragma unroll 1
+  for (; i + 8 <= n; i += 8) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) step(w + (i + u) * WS, x + (i + u) * NT, (i + u) >> 2);
+  }
+#pragma unroll 1
+  for (; i < n; ++i) step(w + i * WS, x + i * NT, i >> 2);
+}
+
+// Width of a weight row in shared memory: what the output groups of dense_tile cover, or one
+// 16-byte load of the output layer.
+constexpr int w_stride(int out, bool output_layer) {
+  return output_layer ? r4(out) : out <= 32 ? 32 : out <= 64 ? 64 : r4(out);
+}
+
+// One hidden layer of a warp's WP pixels, in place in the activation rows.  OG output groups of 4
+// outputs (16 for layers of 33 to 64 outputs, else 8) x 32 / OG pixel groups.
+template <int OG, int WP, int NT>
+__device__ __forceinline__ void dense_tile(const NetLayer& L, const NetSeq& g, const float* __restrict__ W, float* act,
+                                           int lane, int line_px) {
+  constexpr int PX = WP * OG / 32, C = PX / 4;
+  const int px0 = line_px + lane / OG * PX, og = lane & (OG - 1);
+  unsigned long long acc[4][PX / 2];
+#pragma unroll
+  for (int o = 0; o < 4; ++o)
+#pragma unroll
+    for (int c = 0; c < PX / 2; ++c) acc[o][c] = 0ull;
+  const float* w = W + og * 4;
+  int row0 = 0, n = L.mode == 2 ? g.opo : L.in;
+#pragma unroll 1  // one copy of the unrolled rows in the instruction cache
+  for (int left = L.in; left > 0; n = left, row0 = g.aux) {
+    mm_rows<PX, OG * 4, NT>(acc, w, act, row0, n, px0);
+    w += n * (OG * 4);
+    left -= n;
+  }
+  __syncwarp();  // every read of the rows below is done
+  float* dst = act + og * 4 * NT;
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const int at = (((px0 >> 2) ^ (og & 7 & ~(C - 1))) << 2) + ((c ^ (og & (C - 1))) << 2);
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+      float4 v;
+      f2_unpack(acc[o][2 * c], v.x, v.y);
+      f2_unpack(acc[o][2 * c + 1], v.z, v.w);
+      if (L.relu) v = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+      *reinterpret_cast<float4*>(dst + o * NT + at) = v;
+    }
+  }
+  __syncwarp();
+}
+
+// The 3-wide output layer over rows row0 .. row0 + n (row0: a multiple of 32), one pixel per lane.
 template <int NT>
-__global__ void __launch_bounds__(NT, 1) relight_fp32_generic_kernel(Fp32Params p, const __grid_constant__ GenNet g) {
+__device__ __forceinline__ void out_rows(float (&T)[3], const float* __restrict__ w, const float* act, int row0, int n,
+                                         int px) {
+  auto step = [&](const float* wr, const float* xr, int swz) {
+    const float x = xr[(((px >> 2) ^ swz) << 2) + (px & 3)];
+    const float4 v = *reinterpret_cast<const float4*>(wr);
+    T[0] = fmaf(v.x, x, T[0]);
+    T[1] = fmaf(v.y, x, T[1]);
+    T[2] = fmaf(v.z, x, T[2]);
+  };
+  const float* x = act + row0 * NT;
+#pragma unroll 1
+  for (; n >= 32; n -= 32, x += 32 * NT, w += 32 * 4) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) step(w + i * 4, x + i * NT, i >> 2);
+  }
+#pragma unroll 2
+  for (int i = 0; i < n; ++i) step(w + i * 4, x + i * NT, i >> 2);
+}
+
+// NT pixels per block, WP per warp.
+template <int NT, int WP>
+__global__ void __launch_bounds__(NT / WP * 32, 1) relight_fp32_kernel(const __grid_constant__ Fp32Params p,
+                                                                       const __grid_constant__ NetSeq g) {
+  constexpr int kThreads = NT / WP * 32;
   extern __shared__ __align__(16) float sm[];
   float* sW = sm;
   float* sE = sW + p.w_floats;
   float* sL = sE + kMaxKChunk * g.d;
   float* sAct = sL + kMaxKChunk * 4;
-  const int tid = threadIdx.x;
-  for (int i = tid * 4; i < p.w_floats; i += NT * 4)
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int i = tid * 4; i < p.w_floats; i += kThreads * 4)
     *reinterpret_cast<float4*>(sW + i) = __ldg(reinterpret_cast<const float4*>(p.w + i));
-  const int64_t px = p.px_begin + (int64_t)blockIdx.x * NT + tid;
+  // the warp's pixels: WP of a line; lanes beyond WP repeat one and store nothing
+  const int warp_px = (tid >> 5) * WP, line_px = warp_px & 31, lpx = lane & (WP - 1);
+  float* act = sAct + (warp_px & ~31);
+  const int64_t px = p.px_begin + (int64_t)blockIdx.x * NT + warp_px + lpx;
   const bool valid = px < p.n_px;
   const bool active = valid && p.flag[px] != 0;
-  float* act = sAct + tid;
-  if (valid) {
-    const float4* row = reinterpret_cast<const float4*>(p.packed) + px * 4;
-    const float4 r0 = row[0], r1 = row[1], r2 = row[2], r3 = row[3];
-    if (active) hash_encode(p.hl, p.hash, r0.x, r0.y, r0.z, act, NT, g.enc);
-    const float aux13[13] = {r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z, r2.w, r3.x, r3.y, r3.z, r3.w};
-    for (int i = 0; i < g.auxw; ++i) act[(g.aux + i) * NT] = i < 13 ? aux13[i] : 1.0f;
+  const bool warp_active = __any_sync(0xffffffffu, active);
+  if (lane < WP) {
+    // a pixel that is not active is evaluated (with zeros) beside its warp's others, and not summed
+    if (active) {
+      const float4* row = reinterpret_cast<const float4*>(p.packed) + px * 4;
+      const float4 r0 = row[0], r1 = row[1], r2 = row[2], r3 = row[3];
+      hash_encode(p.hl, p.hash, r0.x, r0.y, r0.z,
+                  [&](int i, float v) { act[act_at<NT>(g.enc + i, line_px + lpx)] = v; });
+      const float aux13[13] = {r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z, r2.w, r3.x, r3.y, r3.z, r3.w};
+      for (int i = 0; i < g.auxw; ++i) act[act_at<NT>(g.aux + i, line_px + lpx)] = i < 13 ? aux13[i] : 1.0f;
+    } else {
+      for (int i = 0; i < g.d; ++i) act[act_at<NT>(g.enc + i, line_px + lpx)] = 0.f;
+      for (int i = 0; i < g.auxw; ++i) act[act_at<NT>(g.aux + i, line_px + lpx)] = 0.f;
+    }
   }
   float s[3] = {0.f, 0.f, 0.f}, comp[3] = {0.f, 0.f, 0.f};
   for (int k0 = 0; k0 < p.K; k0 += kMaxKChunk) {
     const int kc = min(kMaxKChunk, p.K - k0);
     __syncthreads();
-    for (int i = tid; i < kc * g.d; i += NT) sE[i] = p.emb_k[(size_t)k0 * g.d + i];
-    for (int i = tid; i < kc * 3; i += NT) sL[(i / 3) * 4 + i % 3] = p.strength[(size_t)k0 * 3 + i];
+    for (int i = tid; i < kc * g.d; i += kThreads) sE[i] = p.emb_k[(size_t)k0 * g.d + i];
+    for (int i = tid; i < kc * 3; i += kThreads) sL[(i / 3) * 4 + i % 3] = p.strength[(size_t)k0 * 3 + i];
     __syncthreads();
-    if (!active) continue;
+    if (!warp_active) continue;
     for (int kk = 0; kk < kc; ++kk) {
-      float T[3];
-      for (int li = 0; li < g.n; ++li)
-        dense_rt<NT>(g.l[li], g, sW + g.l[li].w_off, act, sE + kk * g.d, li + 1 == g.n ? T : nullptr);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        float term = __fmul_rn(sL[kk * 4 + c], T[c]);
-        if (p.clamp) term = fmaxf(term, 0.0f);
-        if (p.kahan) {
-          const float y = __fsub_rn(term, comp[c]);
-          const float t = __fadd_rn(s[c], y);
-          comp[c] = __fsub_rn(__fsub_rn(t, s[c]), y);
-          s[c] = t;
-        } else {
-          s[c] = __fadd_rn(s[c], term);
+      // cp_i = enc_i * E_k,i (ptwise_mlt) into the first rows
+      const float* e = sE + kk * g.d;
+#pragma unroll 8
+      for (int i = lane / WP; i < g.d; i += 32 / WP)
+        act[act_at<NT>(i, line_px + lpx)] = __fmul_rn(act[act_at<NT>(g.enc + i, line_px + lpx)], e[i]);
+      __syncwarp();
+#pragma unroll 1
+      for (int li = 0; li + 1 < g.n; ++li) {
+        const NetLayer& L = g.l[li];
+        if (L.out > 32) dense_tile<16, WP, NT>(L, g, sW + L.w_off, act, lane, line_px);
+        else dense_tile<8, WP, NT>(L, g, sW + L.w_off, act, lane, line_px);
+      }
+      float T[3] = {0.f, 0.f, 0.f};
+      {
+        const NetLayer& L = g.l[g.n - 1];
+        const float* w = sW + L.w_off;
+        int row0 = 0, n = L.mode == 2 ? g.opo : L.in;
+#pragma unroll 1
+        for (int left = L.in; left > 0; n = left, row0 = g.aux) {
+          out_rows<NT>(T, w, act, row0, n, line_px + lpx);
+          w += n * 4;
+          left -= n;
         }
       }
+      if (active) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          float term = __fmul_rn(sL[kk * 4 + c], T[c]);
+          if (p.clamp) term = fmaxf(term, 0.0f);
+          if (p.kahan) {
+            const float y = __fsub_rn(term, comp[c]);
+            const float t = __fadd_rn(s[c], y);
+            comp[c] = __fsub_rn(__fsub_rn(t, s[c]), y);
+            s[c] = t;
+          } else {
+            s[c] = __fadd_rn(s[c], term);
+          }
+        }
+      }
+      __syncwarp();  // the output layer's reads, before the next wavelet's first writes
     }
   }
-  if (valid) {
+  if (valid && lane < WP) {
     const float4 dl = reinterpret_cast<const float4*>(p.direct)[px];
     reinterpret_cast<float4*>(p.indirect)[px] = make_float4(s[0], s[1], s[2], 1.f);
     reinterpret_cast<float4*>(p.with_direct)[px] =
@@ -355,75 +330,63 @@ __global__ void __launch_bounds__(NT, 1) relight_fp32_generic_kernel(Fp32Params 
   }
 }
 
-// The run-time layer sequence of d: out_prd's layers (the first takes the CP product), then
-// cmp_net's (the first takes [out_prd || aux]); the last layer writes T.
-bool gen_net(const NetDims& d, GenNet* g, std::string* why) {
+// The layer sequence of d: out_prd's layers (the first takes the CP product), then cmp_net's
+// (the first takes [out_prd || aux]); the last layer writes T.
+bool net_seq(const NetDims& d, int max_smem, NetSeq* g, std::string* why) {
   auto no = [&](const char* m) { if (why) *why = m; return false; };
-  if (d.op_nl + d.cn_nl > kGenMaxLayers) return no("fp32 relight: too many layers");
+  if (d.op_nl + d.cn_nl > kMaxNetLayers) return no("fp32 relight: too many layers");
   int off = 0, widest = d.op_out;
   for (int i = 0; i < d.op_nl; ++i) {
-    if (d.op_outs[i] > kGenMaxOut) return no("fp32 relight: layer widths above 64 are not supported");
-    g->l[g->n++] = GenLayer{d.op_in[i], d.op_outs[i], i + 1 < d.op_nl ? 1 : 0, i == 0 ? 1 : 0, off};
-    off += d.op_in[i] * r4(d.op_outs[i]);
+    if (d.op_outs[i] > kMaxOut) return no("fp32 relight: layer widths above 64 are not supported");
+    g->l[g->n++] = NetLayer{d.op_in[i], d.op_outs[i], i + 1 < d.op_nl ? 1 : 0, i == 0 ? 1 : 0, off};
+    off += d.op_in[i] * w_stride(d.op_outs[i], false);
     widest = d.op_outs[i] > widest ? d.op_outs[i] : widest;
   }
   for (int i = 0; i < d.cn_nl; ++i) {
-    if (d.cn_outs[i] > kGenMaxOut) return no("fp32 relight: layer widths above 64 are not supported");
-    g->l[g->n++] = GenLayer{d.cn_in[i], d.cn_outs[i], i + 1 < d.cn_nl ? 1 : 0, i == 0 ? 2 : 0, off};
-    off += d.cn_in[i] * r4(d.cn_outs[i]);
+    if (d.cn_outs[i] > kMaxOut) return no("fp32 relight: layer widths above 64 are not supported");
+    g->l[g->n++] = NetLayer{d.cn_in[i], d.cn_outs[i], i + 1 < d.cn_nl ? 1 : 0, i == 0 ? 2 : 0, off};
+    off += d.cn_in[i] * w_stride(d.cn_outs[i], i + 1 == d.cn_nl);
     if (i + 1 < d.cn_nl) widest = d.cn_outs[i] > widest ? d.cn_outs[i] : widest;
   }
   if (d.cn_outs[d.cn_nl - 1] != 3) return no("fp32 relight: cmp_net must end in 3 outputs");
+  // The largest network: its weights beside the activations of 128 pixels, nothing padded.
+  size_t floats = (size_t)kMaxKChunk * (d.enc_dims() + 4) + (size_t)128 * (widest + d.enc_dims() + d.aux_width);
+  for (int i = 0; i < d.op_nl; ++i) floats += (size_t)d.op_in[i] * r4(d.op_outs[i]);
+  for (int i = 0; i < d.cn_nl; ++i) floats += (size_t)d.cn_in[i] * r4(d.cn_outs[i]);
+  if (floats * sizeof(float) > (size_t)max_smem) return no("fp32 relight: network too large for shared memory");
   g->d = d.enc_dims();
   g->opo = d.op_out;
   g->auxw = d.aux_width;
-  g->enc = widest;
-  g->aux = widest + g->d;
-  g->rows = g->aux + g->auxw;
+  if (g->d > widest) widest = g->d;  // the CP product takes the first rows
+  g->aux = (widest + 31) & ~31;
+  g->enc = g->aux + g->auxw;
+  g->rows = g->enc + g->d;
   return true;
 }
 
-size_t gen_smem_bytes(const GenNet& g, int w_floats, int nt) {
+size_t net_smem_bytes(const NetSeq& g, int w_floats, int nt) {
   return sizeof(float) * ((size_t)w_floats + kMaxKChunk * g.d + kMaxKChunk * 4 + (size_t)g.rows * nt);
 }
 
-template <int D, int OPH, int OPO, int CNH, int W, int AUXW>
-bool try_launch(const NetDims& d, const Fp32Params& p, cudaStream_t st) {
-  if (d.enc_dims() != D || d.op_hidden != OPH || d.op_out != OPO || d.cn_hidden != CNH ||
-      d.aux_width != AUXW || (OPH > 0 && d.op_neurons != W) || (CNH > 0 && d.cn_neurons != W))
-    return false;
-  int dev = 0, max_smem = 0;
-  NWPRT_CUDA(cudaGetDevice(&dev));
-  NWPRT_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  using N256 = Net<D, OPH, OPO, CNH, W, AUXW, 256>;
-  using N128 = Net<D, OPH, OPO, CNH, W, AUXW, 128>;
-  if (N256::weight_floats() != p.w_floats) fail(NWPRT_INVALID_ARG, "fp32 weight layout mismatch");
+template <int NT, int WP>
+void launch_nt(const Fp32Params& p, const NetSeq& g, cudaStream_t st) {
+  auto k = relight_fp32_kernel<NT, WP>;
+  const size_t smem = net_smem_bytes(g, p.w_floats, NT);
+  NWPRT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int64_t n = p.n_px - p.px_begin;
-  if (N256::smem_bytes(p.w_floats) <= (size_t)max_smem && n >= 256 * 148) {
-    auto k = relight_fp32_kernel<N256, D, AUXW, 256>;
-    const size_t smem = N256::smem_bytes(p.w_floats);
-    NWPRT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<(unsigned)((n + 255) / 256), 256, smem, st>>>(p);
-  } else {
-    auto k = relight_fp32_kernel<N128, D, AUXW, 128>;
-    const size_t smem = N128::smem_bytes(p.w_floats);
-    if (smem > (size_t)max_smem) fail(NWPRT_UNSUPPORTED, "fp32 relight: network too large for shared memory");
-    NWPRT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<(unsigned)((n + 127) / 128), 128, smem, st>>>(p);
-  }
+  k<<<(unsigned)((n + NT - 1) / NT), NT / WP * 32, smem, st>>>(p, g);
   NWPRT_CUDA(cudaGetLastError());
-  return true;
 }
 
 }  // namespace
 
-// Transposes each row-major [out][in] layer to [in][round4(out)] (zero padded).
+// Transposes each row-major [out][in] layer to [in][w_stride] (zero padded).
 void pack_fp32_weights(const NetDims& d, const float* op, const float* cn, std::vector<float>* op_t,
                        std::vector<float>* cn_t) {
-  auto pack = [](int nl, const int* in, const int* out, const float* src, std::vector<float>* dst) {
+  auto pack = [](int nl, const int* in, const int* out, const float* src, std::vector<float>* dst, bool ends) {
     dst->clear();
     for (int l = 0; l < nl; ++l) {
-      const int o4 = r4(out[l]);
+      const int o4 = w_stride(out[l], ends && l + 1 == nl);
       size_t base = dst->size();
       dst->resize(base + (size_t)in[l] * o4, 0.f);
       for (int j = 0; j < out[l]; ++j)
@@ -431,12 +394,11 @@ void pack_fp32_weights(const NetDims& d, const float* op, const float* cn, std::
       src += (size_t)in[l] * out[l];
     }
   };
-  pack(d.op_nl, d.op_in, d.op_outs, op, op_t);
-  pack(d.cn_nl, d.cn_in, d.cn_outs, cn, cn_t);
+  pack(d.op_nl, d.op_in, d.op_outs, op, op_t, false);
+  pack(d.cn_nl, d.cn_in, d.cn_outs, cn, cn_t, true);
 }
 
-// The two standard shapes run compile-time kernels; every other network whose layers are at
-// most 64 wide (and whose weights fit in shared memory) runs the generic kernel.
+// Any network that net_seq accepts.
 void launch_relight_fp32(const NetDims& d, const HashLevels& hl, const DeviceWeights& w,
                          const RelightJob& job, int clamp, int kahan, cudaStream_t st) {
   if (job.n_px <= job.px_begin) return;
@@ -457,23 +419,43 @@ void launch_relight_fp32(const NetDims& d, const HashLevels& hl, const DeviceWei
   p.with_direct = job.with_direct;
   p.clamp = clamp;
   p.kahan = kahan;
-  if (try_launch<16, 0, 26, 2, 64, 16>(d, p, st)) return;
-  if (try_launch<32, 3, 64, 3, 64, 16>(d, p, st)) return;
-  GenNet g;
-  std::string why;
-  if (!gen_net(d, &g, &why)) fail(NWPRT_UNSUPPORTED, why);
-  const GenLayer& last = g.l[g.n - 1];
-  if (last.w_off + last.in * r4(last.out) != p.w_floats) fail(NWPRT_INVALID_ARG, "fp32 weight layout mismatch");
-  int dev = 0, max_smem = 0;
+  int dev = 0, max_smem = 0, sms = 0;
   NWPRT_CUDA(cudaGetDevice(&dev));
   NWPRT_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const size_t smem = gen_smem_bytes(g, p.w_floats, 128);
-  if (smem > (size_t)max_smem) fail(NWPRT_UNSUPPORTED, "fp32 relight: network too large for shared memory");
-  auto k = relight_fp32_generic_kernel<128>;
-  NWPRT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NWPRT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  NetSeq g;
+  std::string why;
+  if (!net_seq(d, max_smem, &g, &why)) fail(NWPRT_UNSUPPORTED, why);
+  const NetLayer& last = g.l[g.n - 1];
+  if (last.w_off + last.in * w_stride(last.out, true) != p.w_floats) fail(NWPRT_INVALID_ARG, "fp32 weight layout mismatch");
   const int64_t n = p.n_px - p.px_begin;
-  k<<<(unsigned)((n + 127) / 128), 128, smem, st>>>(p, g);
-  NWPRT_CUDA(cudaGetLastError());
+  auto fits = [&](int nt) { return net_smem_bytes(g, p.w_floats, nt) <= (size_t)max_smem; };
+  // Pixels per block (mostly one block per SM at a time, as its weights and activations fill the
+  // shared memory).  Blocks of 256 and more give a warp 32 pixels, smaller ones 16: half the
+  // arithmetic per weight read, twice the warps.  us of one round of 148 blocks at K = 64:
+  //   pixels           64    128    256    384    512
+  //   128x128 network  306    457    826   1136   1498
+  //   1080p network    764   1261   2460   (the last two do not fit)
+  // The launch takes the size whose rounds cost least, by the first row's ratios.
+  struct Form { int nt; double cost; };
+  const Form forms[] = {{512, 1498}, {384, 1136}, {256, 826}, {128, 457}, {64, 306}};
+  int nt = 0;
+  double best = 0;
+  for (const Form& f : forms) {
+    if (!fits(f.nt)) continue;
+    const double c = (double)(((n + f.nt - 1) / f.nt + sms - 1) / sms) * f.cost;
+    if (!nt || c < best) nt = f.nt, best = c;
+  }
+  if (!nt && fits(32)) nt = 32;
+  switch (nt) {
+    case 512: launch_nt<512, 32>(p, g, st); break;
+    case 384: launch_nt<384, 32>(p, g, st); break;
+    case 256: launch_nt<256, 32>(p, g, st); break;
+    case 128: launch_nt<128, 16>(p, g, st); break;
+    case 64: launch_nt<64, 16>(p, g, st); break;
+    case 32: launch_nt<32, 16>(p, g, st); break;
+    default: fail(NWPRT_UNSUPPORTED, "fp32 relight: network too large for shared memory");
+  }
 }
 
 }  // namespace nwprt
