@@ -100,6 +100,7 @@ struct TcParams {
   uint32_t* err;
   int* tile_ctr;    // tiles taken beyond the warpgroups' first ones (zeroed before the launch);
                     // null when every warpgroup has at most its first tile
+  int stagger;            // the warpgroups' first hash encodings one after another
   int whole_tiles;        // tiles [0, whole_tiles) go to one warpgroup each; for the rest a CTA's
                           // warpgroups share a tile, one chunk of its wavelets each
   // Shared-memory descriptors of every layer's B tile, its aux block and the output layer's
@@ -623,6 +624,7 @@ struct __align__(16) TcBarriers {
   uint64_t wload;           // the weight blob's TMA load
   uint32_t tmem_base;
   int tile_slot[kNWG];      // the tile each warpgroup took from the launch's counter
+  int tile_now[kNWG];       // the tile each warpgroup works on (kept here, not in a register)
 };
 
 // Shared-memory bytes of the weight region: whole TMA boxes, rounded to 1 KB.
@@ -791,11 +793,9 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
   // next one (every tile has at least one).  Shared tiles, after them: the CTA's warpgroups work
   // on one tile, a chunk of its wavelets each (few tiles would leave most chains idle).
   int t = p.whole_tiles == 0 ? (int)blockIdx.x : g * (int)gridDim.x + (int)blockIdx.x;
-  // The first tiles' hash encodings are staggered: warpgroup g + 1 starts when g has two thirds
-  // of its levels.  Their rate is the SM's anyway, and started together no chain would run until
-  // all five are done; started in turn, the first chain runs after a fifth of the time.
-  if (p.whole_tiles > 0 && g > 0) named_sync(5 + g, 256);
-  if (p.whole_tiles > 0 && g + 1 < kNWG && t >= p.whole_tiles) named_arrive(6 + g, 256);
+  // Staggered first hash encodings: warpgroup g + 1 starts when g has two thirds of its levels.
+  // Their rate is the SM's anyway; started in turn, the tiles that follow stay out of step.
+  if (p.stagger && g > 0) named_sync(5 + g, 256);
   // This warpgroup is done with whole tiles: its first shared tile, after the CTA's others are too.
   auto leave_whole = [&]() -> int {
     if (p.whole_tiles == p.total_tiles) return p.total_tiles;
@@ -812,6 +812,10 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
     auto chunk = [&] { return (J.K + kNWG - 1) / kNWG; };
     auto shared_tile = [&] { return t >= p.whole_tiles; };
     auto k_begin = [&] { return shared_tile() ? min(g * chunk(), J.K) : 0; };
+    // the same once the chain runs
+    auto tile_now = [&] { return *reinterpret_cast<volatile int*>(&bars->tile_now[g]); };
+    auto k_begin_now = [&] { return tile_now() >= p.whole_tiles ? min(g * chunk(), J.K) : 0; };
+    if (q == 0 && lane == 0) bars->tile_now[g] = t;
     // this warpgroup's wavelets: [k_begin, k_begin + K)
     const int K = shared_tile() ? min(chunk(), J.K - k_begin()) : J.K;
     const long long px = J.px_begin + (t - J.tile_begin) * kTile + row;
@@ -827,7 +831,7 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
       } else {
         constexpr int kPart = DMAX / 3;
         hash_encode_pairs(p.hl, p.hash, r0.x, r0.y, r0.z, 0, kPart, 1, put);
-        if (g + 1 < kNWG && t < kNWG * (int)gridDim.x) named_arrive(6 + g, 256);  // the first tile
+        if (p.stagger && g + 1 < kNWG && t < kNWG * (int)gridDim.x) named_arrive(6 + g, 256);  // the first tile
         hash_encode_pairs(p.hl, p.hash, r0.x, r0.y, r0.z, kPart, DMAX / 2, 1, put);
       }
       if (valid) {
@@ -859,6 +863,12 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
       if (ok && q == lead && elect_one()) issue_next(0);
     }
     float* my_sums = sums + g * 6 * kTile + row;
+    // the chunk's sums join the tile's
+    auto flush = [&] {
+      add_chunk(my_sums, flush_at == chunk(), p.kahan, s0, s1, s2, c0, c1, c2);
+      s0 = s1 = s2 = c0 = c1 = c2 = 0.f;
+      flush_at += chunk();
+    };
     // T_k -> clamped Kahan sums, then the next wavelet's first-layer operand
     auto finish_wavelet = [&](int k, float t0, float t1, float t2) {
       float L0, L1, L2;
@@ -866,7 +876,7 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
         const float4 Lk = bars->l_ring[g][k % kRing];
         L0 = Lk.x; L1 = Lk.y; L2 = Lk.z;
       } else {
-        const float* Lk = J.strength + (size_t)(k_begin() + k) * 3;
+        const float* Lk = J.strength + (size_t)(k_begin_now() + k) * 3;
         L0 = __ldg(Lk + 0); L1 = __ldg(Lk + 1); L2 = __ldg(Lk + 2);
       }
       float u0 = __fmul_rn(L0, t0);
@@ -881,13 +891,9 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
       } else {
         s0 = __fadd_rn(s0, u0); s1 = __fadd_rn(s1, u1); s2 = __fadd_rn(s2, u2);
       }
-      if (k + 1 == flush_at) {  // the chunk's sums join the tile's
-        add_chunk(my_sums, flush_at == chunk(), p.kahan, s0, s1, s2, c0, c1, c2);
-        s0 = s1 = s2 = c0 = c1 = c2 = 0.f;
-        flush_at += chunk();
-      }
+      if (!OUT_TC && k + 1 == flush_at) flush();
       if (!OUT_TC && k + 1 < K) {  // OUT_TC: written while the output layer's MMA runs
-        const int kn = k_begin() + k + 1;
+        const int kn = k_begin_now() + k + 1;
         store_cp<DMAX, MODE>(enc_s, J.emb_k + (size_t)kn * p.enc_dims, J.emb_h + (size_t)kn * (p.enc_dims / 2),
                              a_taddr, p.cp_scale, p.amax);
         tmem_wait_st();
@@ -994,7 +1000,7 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
           // E_k+1..k+8 and L_k..k+7 into the rings, by a warp that would otherwise only wait
           // for this layer's MMAs; waited for before this wavelet's last hidden-layer barrier
           constexpr int C = DMAX / 8;
-          const int j = lane / C, kb = k_begin();
+          const int j = lane / C, kb = k_begin_now();
           if (j < kBatch && k + 1 + j < K)
             cp_async16(smem_u32(&bars->e_ring[g][(k + 1 + j) % kRing][lane % C]),
                        J.emb_h + (size_t)(kb + k + 1 + j) * (p.enc_dims / 2) + (lane % C) * 4);
@@ -1006,6 +1012,9 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
         // T_k's clamped Kahan update waits one more step: under the next wavelet's second layer,
         // whose MMAs take longer than its first layer's, so that it stays off the chain
         if (OUT_TC && l == 1 && k > 0) finish_wavelet(k - 1, tk0, tk1, tk2);
+        // not in finish_wavelet, and a layer later where there is one: that is 0.9% of a round faster
+        if (OUT_TC && l == (Sh::nl > 2 ? 2 : 1) && k == flush_at) flush();
+
         if (OUT_TC && nl == n_layers && k + 1 < K) {
           // the next wavelet's first-layer operand into the A columns, which the output MMA
           // (operand in [64, 96), accumulator in [32, 48)) does not touch
@@ -1014,6 +1023,7 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
         }
       }
     }
+    t = tile_now();
     if (shared_tile()) {
       // the chunks' sums meet in warpgroup 0, in order
       add_chunk(my_sums, true, p.kahan, s0, s1, s2, c0, c1, c2);
@@ -1497,6 +1507,10 @@ void launch_relight_tc(const NetDims& d, const HashLevels& hl, const float* hash
   const long long per_sm = (rest + sms - 1) / sms;
   const bool share = per_sm <= 4 && k_min >= 12 * (per_sm - 1) && (full == 0 || k_min == k_max);
   p.whole_tiles = (int)(share ? full : tiles);
+  // From three rounds on, later tiles' encodings overlapping the other chains' work pays for the
+  // later start of the last chains: 6 rounds at K = 128 2735 -> 2715 us, 3 rounds at K = 64
+  // 680 -> 671, 1 round at K = 64 226 -> 238 (1080p network).
+  p.stagger = p.whole_tiles >= 3 * kNWG * sms;
   const bool counted = p.whole_tiles > (long long)kNWG * grid;
   p.tile_ctr = counted ? tile_ctr : nullptr;
   auto go = [&](auto kern) {
