@@ -6,8 +6,8 @@
 // is a non-decreasing step function of x with 255 steps.  The host finds each step's
 // threshold once -- the smallest float whose byte reaches j, by bisection over the ordered
 // bit patterns of non-negative floats, evaluating srgb_byte itself -- and the kernel maps a
-// channel to the number of thresholds at or below it (an estimate, then one or two exact
-// comparisons in shared memory).
+// channel to the number of thresholds at or below it (an estimate, then one exact comparison in
+// shared memory).
 // That equals srgb_byte wherever srgb_byte is monotonic, which the oracle checks float by
 // float around every threshold.  One float4 read and one 32-bit write per pixel: HBM-bound.
 #include <mutex>
@@ -43,40 +43,32 @@ const SrgbTable& table() {
   return T;
 }
 
-constexpr int kPix = 2;  // pixels per thread per iteration
-
-// Number of thresholds at or below x.  A fast estimate (the SFU power) lands within a step or
-// two of the answer; walking the exact thresholds from there makes the result independent of
-// the estimate's accuracy.  NaN and negative x give 0, +inf gives 255.
+// Number of thresholds at or below x.  The estimate g (the SFU power) is within 0.01 of the real
+// step position: with x + 1e-6 >= 1e-6, lg2.approx is off by at most 3 ulp of 20, so the power by
+// 2e-6 of itself and g, at most 271, by 6e-4, far below 1/2.  So the count is floor(g - 1/2) or one
+// more, and one exact comparison decides.  NaN and negative x give 0, +inf gives 255.
 __device__ __forceinline__ uint32_t lookup(const float* t, float x) {
   const float g = fmaf(1.055f, __powf(fmaxf(x, 0.f) + 1e-6f, 1.0f / 2.4f), -0.055f) * 255.9f;
-  int j = g > 0.f ? (g < 255.f ? (int)g : 255) : 0;
-  while (j < 255 && t[j + 1] <= x) ++j;
-  while (j > 0 && !(t[j] <= x)) --j;
-  return (uint32_t)j;
+  const int j = (int)fminf(fmaxf(g - 0.5f, 0.f), 254.f);
+  return (uint32_t)j + (t[j + 1] <= x ? 1u : 0u);
 }
 
+// HBM-bound.  A shared-memory lookup of a pseudo-random threshold meets a 3-way bank conflict, so
+// one lookup per channel instead of three to four, and the table's load off the constant bank, took
+// 16 1080p frames from 160 to 103 us (6,440 GB/s) and one 2559 x 1439 frame from 23.6 to 14.2 us.
+// One pixel per thread and iteration on 8 blocks per SM (every thread slot): 2 or 4 pixels measured
+// 16.8 and 17.4 us on that frame, 64 blocks per SM 18.1 us (100 us on the 16 frames).
 __global__ void __launch_bounds__(256) tonemap_srgb_kernel(const __grid_constant__ SrgbTable T,
                                                            const float4* __restrict__ src, int64_t n,
                                                            uint32_t* __restrict__ dst) {
   __shared__ float t[256];
-  t[threadIdx.x] = T.t[threadIdx.x];
+  const float* table = T.t;
+  asm volatile("" : "+l"(table));  // one coalesced load, not 32 constant-bank reads per warp
+  t[threadIdx.x] = table[threadIdx.x];
   __syncthreads();
-  // a block covers kPix * 256 consecutive pixels per iteration; each thread keeps kPix
-  // coalesced loads in flight before the lookups
-  const int64_t span = (int64_t)kPix * blockDim.x;
-  for (int64_t base = (int64_t)blockIdx.x * span + threadIdx.x; base < n; base += (int64_t)gridDim.x * span) {
-    float4 v[kPix];
-#pragma unroll
-    for (int k = 0; k < kPix; ++k) {
-      const int64_t i = base + (int64_t)k * blockDim.x;
-      if (i < n) v[k] = __ldg(src + i);
-    }
-#pragma unroll
-    for (int k = 0; k < kPix; ++k) {
-      const int64_t i = base + (int64_t)k * blockDim.x;
-      if (i < n) dst[i] = lookup(t, v[k].x) | (lookup(t, v[k].y) << 8) | (lookup(t, v[k].z) << 16) | (255u << 24);
-    }
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const float4 v = __ldg(src + i);
+    dst[i] = lookup(t, v.x) | (lookup(t, v.y) << 8) | (lookup(t, v.z) << 16) | (255u << 24);
   }
 }
 
@@ -91,8 +83,7 @@ void launch_tonemap_srgb(const float* src, int64_t n, uint32_t* dst, cudaStream_
   int dev = 0, sms = 0;
   NWPRT_CUDA(cudaGetDevice(&dev));
   NWPRT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int64_t blocks = (n + kPix * 256 - 1) / (kPix * 256);
-  const int64_t cap = (int64_t)sms * 64;  // measured: 8 -> 64 blocks per SM took 16 frames from 193 to 164 us
+  const int64_t blocks = (n + 255) / 256, cap = (int64_t)sms * 8;
   tonemap_srgb_kernel<<<(int)(blocks < cap ? blocks : cap), 256, 0, st>>>(
       table(), reinterpret_cast<const float4*>(src), n, dst);
   NWPRT_CUDA(cudaGetLastError());
