@@ -8,14 +8,23 @@
 // projects it by sampling its material callables, devicePrograms.cu:448-474; here it is an
 // input like T).  Per pixel: (1-u-v) c[i0] + u c[i1] + v c[i2].
 //
-// The vertex pass streams T once and does 2 n^2 FMAs per 4 n^2 bytes: HBM-bound.  One warp
-// per vertex: the warp copies T[v] and brdf[v] into shared memory with cp.async, all copies
-// in flight at once.  T[v] starts 4 (v mod 4) bytes past a 16-byte boundary (n^2 = 6561 is
-// odd), so the staging base is shifted by the same amount and the body moves in 16-byte
-// copies, with a head and a tail of at most three 4-byte copies.  Then lane k walks row k
-// sequentially (so the sum order is the reference's).  The row stride n = 81 is odd, so the
-// 32 lanes read 32 different banks.  Eight warps per SM overlap one vertex's copy with
-// another's arithmetic.
+// The vertex pass streams T once and does 2 n^2 FMAs per 4 n^2 bytes: HBM-bound.  One warp per
+// vertex, eight per CTA: the warp copies T[v] into its shared-memory stage (bulk copies, tracked
+// by an mbarrier) and brdf[v] beside it, then lane k walks rows k, k + 32, k + 64 side by side,
+// each sequentially (so the sum order is the reference's), one lane per channel sums over k, and
+// the other warps' copies run meanwhile.  How the rows sit in the stage:
+//  * odd n: as in memory, the odd stride being free of bank conflicts.  T[v] starts 4 (v n^2 mod
+//    4) bytes past a 16-byte boundary, so the stage is shifted by as much: the body moves in one
+//    bulk copy, a head and a tail of at most three floats by cp.async.
+//  * n a multiple of 4, T 16-byte aligned: rows an odd number of 16-byte chunks apart, read four
+//    terms at a time.  One bulk copy where n / 4 is odd, else one per row.
+//  * otherwise: an odd stride, by 4-byte cp.async.
+// 40,000 vertices of 81 coefficients: 249 us with one row at a time (three env SH reads per term
+// and row) and 16-byte cp.async, 201 with three rows side by side, 157 with bulk copies (6,930
+// GB/s); 14,364 of 64: 277 us (32-way conflicts), 148 by 4-byte copies to an odd stride, 67 by
+// rows; 16,146 of 25: 27.3 -> 13 us, as many CTAs per SM as fit instead of one.
+#include <type_traits>
+
 #include "nwprt_internal.cuh"
 
 namespace nwprt {
@@ -24,69 +33,125 @@ namespace {
 constexpr int kMaxN = 81;
 constexpr int kWarps = 8;
 
-// Shared memory in floats: env SH, then per warp light[k] and brdf[v] ([kMaxN][3] each), then
-// per warp a T staging area of n^2 floats plus up to 3 of alignment shift, rounded to 16 bytes.
-__host__ __device__ constexpr int stage_offset() { return ((1 + 2 * kWarps) * kMaxN * 3 + 3) & ~3; }
-__host__ __device__ constexpr int stage_stride(int n) { return (n * n + 3 + 3) & ~3; }
+enum RowForm { kOddRows, kChunkRows, kSingles };  // how a matrix is staged (above)
 
+// Shared memory in floats: the env SH (padded to 4 per coefficient), then per warp light[k] and
+// brdf[v] ([kMaxN][3] each), then per warp a T staging area plus up to 3 of alignment shift,
+// rounded to 16 bytes.
+__host__ __device__ constexpr int stage_offset() { return (4 * kMaxN + 2 * kWarps * kMaxN * 3 + 3) & ~3; }
+__host__ __device__ constexpr int row_stride(int n, RowForm form) {
+  return form == kChunkRows ? ((n / 4) | 1) * 4 : n | 1;
+}
+__host__ __device__ constexpr int stage_stride(int n, RowForm form) { return (n * row_stride(n, form) + 3 + 3) & ~3; }
+
+__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+// R = ceil(n / 32): rows per lane.
+template <int R, RowForm FORM>
 __global__ void __launch_bounds__(kWarps * 32) sh_vertex_kernel(const float* __restrict__ T,
                                                                 const float* __restrict__ brdf,
                                                                 const float* __restrict__ L, int64_t V, int n,
                                                                 float* __restrict__ out) {
   extern __shared__ __align__(16) float smem[];
-  const int nn = n * n;
+  __shared__ uint64_t full[kWarps];
+  const int nn = n * n, stride = row_stride(n, FORM);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* sL = smem;                                              // [kMaxN][3] env SH
-  float* light = smem + (1 + warp) * kMaxN * 3;                  // [kMaxN][3] this warp's light[k]
-  float* sb = smem + (1 + kWarps + warp) * kMaxN * 3;            // [kMaxN][3] this warp's brdf[v]
-  float* stage = smem + stage_offset() + warp * stage_stride(n);  // this warp's T staging (16-byte aligned)
-  for (int i = threadIdx.x; i < n * 3; i += blockDim.x) sL[i] = L[i];
+  float4* sL = reinterpret_cast<float4*>(smem);                         // [kMaxN] env SH
+  float* light = smem + 4 * kMaxN + warp * kMaxN * 3;                   // [kMaxN][3] this warp's light[k]
+  float* sb = smem + 4 * kMaxN + (kWarps + warp) * kMaxN * 3;           // [kMaxN][3] this warp's brdf[v]
+  float* stage = smem + stage_offset() + warp * stage_stride(n, FORM);  // this warp's T (16-byte aligned)
+  for (int i = threadIdx.x; i < n; i += blockDim.x) sL[i] = make_float4(L[i * 3], L[i * 3 + 1], L[i * 3 + 2], 0.f);
+  if (threadIdx.x < kWarps) mbar_init(&full[threadIdx.x], 1);
+  fence_barrier_init();
   __syncthreads();
+  uint32_t parity = 0;
   for (int64_t v = (int64_t)blockIdx.x * kWarps + warp; v < V; v += (int64_t)gridDim.x * kWarps) {
     const float* src = T + v * nn;
     const float* bsrc = brdf + v * n * 3;
-    // t[i] and src[i] share their offset modulo 16 bytes
-    const int mis = (int)((reinterpret_cast<uintptr_t>(src) >> 2) & 3);
-    float* t = stage + mis;
-    const int head = ((4 - mis) & 3) < nn ? ((4 - mis) & 3) : nn;
-    const int body = (nn - head) & ~3;
-    if (lane < head)
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(t + lane)), "l"(src + lane) : "memory");
-    for (int i = head + 4 * lane; i < head + body; i += 128)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(t + i)), "l"(src + i) : "memory");
-    for (int i = head + body + lane; i < nn; i += 32)
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(t + i)), "l"(src + i) : "memory");
+    float* t = stage;
+    if constexpr (FORM == kOddRows) {
+      // t[i] and src[i] share their offset modulo 16 bytes
+      const int mis = (int)((reinterpret_cast<uintptr_t>(src) >> 2) & 3);
+      t += mis;
+      const int head = ((4 - mis) & 3) < nn ? ((4 - mis) & 3) : nn;
+      const int body = (nn - head) & ~3;
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&full[warp], body * 4);
+        if (body > 0) bulk_g2s(t + head, src + head, body * 4, &full[warp]);
+      }
+      if (lane < head) cp_async4(t + lane, src + lane);
+      if (head + body + lane < nn) cp_async4(t + head + body + lane, src + head + body + lane);
+    } else if constexpr (FORM == kChunkRows) {
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&full[warp], nn * 4);
+        if (stride == n) bulk_g2s(t, src, nn * 4, &full[warp]);
+      }
+      __syncwarp();  // the expected bytes are set before a row can complete
+      if (stride != n)
+        for (int r = lane; r < n; r += 32) bulk_g2s(t + r * stride, src + r * n, n * 4, &full[warp]);
+    } else {
+      for (int r = 0; r < n; ++r)
+        for (int c = lane; c < n; c += 32) cp_async4(t + r * stride + c, src + r * n + c);
+    }
     for (int i = lane; i < n * 3; i += 32)
       asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(sb + i)), "l"(bsrc + i) : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncwarp();
-    // lane k owns rows k, k+32, k+64: light[k] = sum_j T[k][j] L[j], j ascending
-    for (int k = lane; k < n; k += 32) {
-      float l0 = 0.f, l1 = 0.f, l2 = 0.f;
-      const float* row = t + k * n;
-      for (int j = 0; j < n; ++j) {
-        const float tj = row[j];
-        l0 = fmaf(tj, sL[j * 3 + 0], l0);
-        l1 = fmaf(tj, sL[j * 3 + 1], l1);
-        l2 = fmaf(tj, sL[j * 3 + 2], l2);
-      }
-      light[k * 3] = l0;
-      light[k * 3 + 1] = l1;
-      light[k * 3 + 2] = l2;
+    if constexpr (FORM != kSingles) {
+      if (!mbar_wait(&full[warp], parity, nullptr)) return;
+      parity ^= 1u;
     }
     __syncwarp();
-    // c = | sum_k light[k] * brdf[k] |, k ascending
-    if (lane == 0) {
-      float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-      for (int k = 0; k < n; ++k) {
-        s0 = fmaf(light[k * 3], sb[k * 3 + 0], s0);
-        s1 = fmaf(light[k * 3 + 1], sb[k * 3 + 1], s1);
-        s2 = fmaf(light[k * 3 + 2], sb[k * 3 + 2], s2);
+    // light[k] = sum_j T[k][j] L[j], j ascending (each env SH term read once for the R rows).
+    // Rows past the last repeat it.
+    float l[R][3];
+    const float* row[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      l[r][0] = l[r][1] = l[r][2] = 0.f;
+      row[r] = t + min(lane + 32 * r, n - 1) * stride;
+    }
+    auto term = [&](int r, float tj, const float4& Lj) {
+      l[r][0] = fmaf(tj, Lj.x, l[r][0]);
+      l[r][1] = fmaf(tj, Lj.y, l[r][1]);
+      l[r][2] = fmaf(tj, Lj.z, l[r][2]);
+    };
+    if constexpr (FORM == kChunkRows) {
+      for (int j = 0; j < n; j += 4) {
+        float4 q[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) q[r] = *reinterpret_cast<const float4*>(row[r] + j);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 Lj = sL[j + i];
+#pragma unroll
+          for (int r = 0; r < R; ++r) term(r, i == 0 ? q[r].x : i == 1 ? q[r].y : i == 2 ? q[r].z : q[r].w, Lj);
+        }
       }
-      out[v * 3 + 0] = fabsf(s0);
-      out[v * 3 + 1] = fabsf(s1);
-      out[v * 3 + 2] = fabsf(s2);
+    } else {
+#pragma unroll 4
+      for (int j = 0; j < n; ++j) {
+        const float4 Lj = sL[j];
+#pragma unroll
+        for (int r = 0; r < R; ++r) term(r, row[r][j], Lj);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (lane + 32 * r < n) {
+        float* d = light + (lane + 32 * r) * 3;
+        d[0] = l[r][0];
+        d[1] = l[r][1];
+        d[2] = l[r][2];
+      }
+    __syncwarp();
+    // c = | sum_k light[k] * brdf[k] |, k ascending, one lane per channel
+    if (lane < 3) {
+      float s = 0.f;
+      for (int k = 0; k < n; ++k) s = fmaf(light[k * 3 + lane], sb[k * 3 + lane], s);
+      out[v * 3 + lane] = fabsf(s);
     }
     __syncwarp();
   }
@@ -123,11 +188,24 @@ void launch_sh_vertex(const float* T, const float* brdf, const float* L, int64_t
   int dev = 0, sms = 0;
   NWPRT_CUDA(cudaGetDevice(&dev));
   NWPRT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const size_t smem = (size_t)(stage_offset() + kWarps * stage_stride(n)) * sizeof(float);
-  NWPRT_CUDA(cudaFuncSetAttribute(sh_vertex_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int64_t blocks = (V + kWarps - 1) / kWarps;
-  const int64_t cap = (int64_t)sms;  // one 8-warp CTA per SM at n = 81 (227 KB of staging)
-  sh_vertex_kernel<<<(int)(blocks < cap ? blocks : cap), kWarps * 32, smem, st>>>(T, brdf, L, V, n, out);
+  auto go = [&](auto kern, RowForm form) {
+    const size_t smem = (size_t)(stage_offset() + kWarps * stage_stride(n, form)) * sizeof(float);
+    NWPRT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;  // 1 at n = 81 (227 KB of staging), up to 8 for few coefficients
+    NWPRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWarps * 32, smem));
+    const int64_t blocks = (V + kWarps - 1) / kWarps, cap = (int64_t)sms * (per_sm > 0 ? per_sm : 1);
+    kern<<<(int)(blocks < cap ? blocks : cap), kWarps * 32, smem, st>>>(T, brdf, L, V, n, out);
+  };
+  auto rows = [&](auto form) {
+    constexpr RowForm F = decltype(form)::value;
+    if (n <= 32) go(sh_vertex_kernel<1, F>, F);
+    else if (n <= 64) go(sh_vertex_kernel<2, F>, F);
+    else go(sh_vertex_kernel<3, F>, F);
+  };
+  // every row of a T[v] starts on a 16-byte boundary if T does and n is a multiple of 4
+  if (n % 2) rows(std::integral_constant<RowForm, kOddRows>{});
+  else if (n % 4 == 0 && (reinterpret_cast<uintptr_t>(T) & 15) == 0) rows(std::integral_constant<RowForm, kChunkRows>{});
+  else rows(std::integral_constant<RowForm, kSingles>{});
   NWPRT_CUDA(cudaGetLastError());
 }
 

@@ -1,0 +1,26 @@
+"""GPU tests of the per-vertex SH kernel's staging forms, bit for bit against the oracle: odd
+coefficient counts (one bulk copy), multiples of 4 (rows of 16-byte chunks, with and without
+padding), the other even ones, and transfer matrices that start on no 16-byte boundary."""
+import numpy as np
+import pytest
+
+from neural_wavelet_prt_demo_b200 import synth
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 6, 8, 16, 25, 31, 32, 33, 36, 49, 62, 64, 65, 72, 80, 81])
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+def test_sh_vertex_forms_bit_exact(cuda, n, shift):
+    import torch
+    from neural_wavelet_prt_demo_b200 import engine as eng
+    V = 19
+    T, brdf, _, _ = synth.make_sh_mesh(V, 1, 81, seed=n)
+    T, brdf = T[:, :n, :n].copy(), brdf[:, :n].copy()
+    L = synth.make_sh_transport(3, 81, seed=5).T[:n].copy()
+    buf = torch.empty(T.size + shift, dtype=torch.float32, device=cuda)
+    Td = buf[shift:].view(V, n, n)
+    Td.copy_(torch.from_numpy(T))
+    got = eng.sh_vertex_radiance(Td, *(torch.from_numpy(a).to(cuda) for a in (brdf, L))).cpu().numpy()
+    assert np.array_equal(got.view(np.uint32), O.sh_vertex_radiance(T, brdf, L).view(np.uint32))
