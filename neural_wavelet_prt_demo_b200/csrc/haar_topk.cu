@@ -1,5 +1,5 @@
 // Cubemap Haar transform + top-K wavelet selection: one thread-block cluster per env map for
-// single maps and small batches, one persistent CTA per map for batches of 32 maps or more
+// single maps and small batches, one persistent CTA per map for batches of 97 maps or more
 // (haar_topk_batch_kernel, described where it is defined).
 //
 // The reference only loads precomputed results (waveletcoeffs/<name>.npy and
@@ -22,15 +22,17 @@
 //    the last levels the same way: one block barrier for the whole transform.  The
 //    coefficients of those upper levels fill exactly the top-left (S/4)^2 block of the
 //    face, one per thread, so each thread owns 16 coefficients.
-//  * 4-pass 8-bit radix select of the K-th largest key over the cluster: each CTA
-//    histograms its keys (registers -> shared atomics), the six histograms are summed
-//    through distributed shared memory after one cluster barrier, and one block scan over
-//    the totals (thread t = digit 255 - t) finds the digit.
-//  * Ties at the threshold are ranked by flat index with a per-face bitmap and popcount
-//    prefixes; the per-face tie counts come from the last pass's histograms.
-//  * Winners get slots from one counter in CTA 0 (one atomic per warp) and are written to
-//    all six CTAs, so each CTA ranks a sixth of them (one warp per winner) and writes
-//    their outputs.
+//  * The bin of the K-th largest key, in a window of 16 binades below the map's largest key at
+//    1/16 binade: each CTA histograms its keys (registers -> shared atomics), and every CTA sums
+//    the six histograms through distributed shared memory.  Two cluster barriers (the maximum,
+//    the histograms), where a radix select over the keys took one per pass of four.
+//  * The keys of that bin and above are listed in all six CTAs, bin by bin, and each CTA ranks its
+//    own face's among their bin's (a few dozen) and writes those of rank below K: one barrier.
+//  * Maps whose window holds fewer than K keys, or more than 512 too many in the last bin (ties),
+//    take a 4-pass 8-bit radix select; ties at the threshold are then ranked by flat index with a
+//    per-face bitmap and popcount prefixes, and every CTA ranks a sixth of the winners.
+// One 6 x 64 x 64 map, graph launches: K = 64 10.6 -> 5.7 us, K = 300 14.2 -> 6.8, K = 1024
+// 25.0 -> 9.8 (radix select for all maps, all-pairs ranking, before).
 #include <cooperative_groups.h>
 
 #include <mutex>
@@ -52,20 +54,28 @@ struct Winner {
   int32_t idx;
 };
 
+// Coefficients the cluster form lists and ranks directly: the K winners and up to 512 more that
+// share the last one's bin.
+__host__ __device__ constexpr int list_cap(int K) { return K + 512; }
+
 struct HaarSmem {
-  uint32_t* hist;    // [2][256] this face's histogram of the pass (double buffered)
+  uint32_t* hist;    // [2][256] this face's histogram: of the window; general form: of a pass (double buffered)
+  uint32_t* seg;     // [256] a window bin's part of the list: start | length << 16
+  uint32_t* cur;     // [256] where this face's next key of the bin goes
+  uint32_t* kmax;    // [6 * kWarps] every warp's largest key
   float* upper;      // [(S/4)^2][3] coefficients of the top-left (S/4)^2 block
   float* llg;        // [16][3] LL values handed to warp 0 for the last levels
   uint32_t* bits;    // [S*S/32] ties at the threshold, by flat index within the face
   uint32_t* wpre;    // [S*S/32] exclusive popcount prefix of `bits`
-  uint64_t* gkey;    // [K] composite keys of the winners (every CTA holds all of them)
-  Winner* gval;      // [K]
+  uint64_t* gkey;    // [list_cap(K)] composite keys of the listed coefficients (in every CTA)
+  Winner* gval;      // [list_cap(K)] the values of this face's; general form: of all K winners
   int* warp_tot;     // [kWarps]
   int* scal;         // scalars
 };
 
 // scal[] slots
 constexpr int kScPrefix = 0, kScMask = 1, kScRemaining = 2, kScCounter = 3, kScEq = 8;  // eq: [6]
+constexpr int kScListed = 14;                // cluster form: keys listed
 constexpr int kScNAbove = 16, kScNCand = 17;  // batched kernel: winners above the window bin, candidates in it
 // Candidates (keys in the window's selected bin) the batched kernel ranks directly; they share
 // the histogram region: composite keys (8 B) + ids (4 B).
@@ -79,16 +89,22 @@ __host__ __device__ inline size_t smem_layout(int S, int K, char* base, HaarSmem
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o = align16(o + bytes); return at; };
   size_t oH = take(sizeof(uint32_t) * 512);
+  size_t oS2 = take(sizeof(uint32_t) * 256);
+  size_t oC2 = take(sizeof(uint32_t) * 256);
+  size_t oM = take(sizeof(uint32_t) * 6 * kWarps);
   size_t oU = take(sizeof(float) * 3 * G * G);
   size_t oL = take(sizeof(float) * 3 * 16);
   size_t oB = take(sizeof(uint32_t) * nw);
   size_t oP = take(sizeof(uint32_t) * nw);
-  size_t oG = take(sizeof(uint64_t) * K);
-  size_t oV = take(sizeof(Winner) * K);
+  size_t oG = take(sizeof(uint64_t) * list_cap(K));
+  size_t oV = take(sizeof(Winner) * list_cap(K));
   size_t oW = take(sizeof(int) * kWarps);
   size_t oS = take(sizeof(int) * 32);
   if (L) {
     L->hist = (uint32_t*)(base + oH);
+    L->seg = (uint32_t*)(base + oS2);
+    L->cur = (uint32_t*)(base + oC2);
+    L->kmax = (uint32_t*)(base + oM);
     L->upper = (float*)(base + oU);
     L->llg = (float*)(base + oL);
     L->bits = (uint32_t*)(base + oB);
@@ -414,8 +430,7 @@ __device__ __forceinline__ void haar_face_in_registers(const float* __restrict__
 }
 
 template <int S>
-// Two CTAs per SM at most: this form serves batches under kBatchMinMaps (at most 186 CTAs
-// on 148 SMs), and the bound leaves the transform its registers (three per SM spilled).
+// Two CTAs per SM at most: the bound leaves the transform its registers (three per SM spilled).
 __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
     haar_topk_kernel(const float* __restrict__ faces, int K, int32_t* __restrict__ idx_out,
                      float* __restrict__ st_out) {
@@ -436,6 +451,9 @@ __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
 
   if (face == 0 && tid == 0) sm.scal[kScCounter] = 0;  // winner slots (read after 5 cluster barriers)
   for (int w = tid; w < NW; w += kThreads) sm.bits[w] = 0u;
+  sm.hist[tid] = 0u;                     // kThreads == 256 bins
+  if (tid == 0) sm.scal[kScListed] = -1;  // stays when the window holds fewer than K keys
+  // (barriers in the transform order these)
 
   // ---- the transform: levels 1-2 in registers, the rest by shuffles and warp 0
   float co[NR > 0 ? NR : 1][3];  // detail coefficients held in registers (RGB)
@@ -454,7 +472,91 @@ __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
   }
   key[NR] = wavelet_key_bits(ur, ug, ub);
 
-  // ---- 4-pass radix select of the K-th largest key over the whole cluster
+  // ---- the map's largest key: every warp's to all six CTAs
+  {
+    uint32_t m = 0;
+    if (owner)
+#pragma unroll
+      for (int u = 0; u < NK; ++u) m = max(m, key[u]);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane < 6) cluster.map_shared_rank(sm.kmax, lane)[face * kWarps + warp] = m;
+  }
+  cluster.sync();
+  uint32_t kmax = sm.kmax[lane];
+  if (lane < 6 * kWarps - 32) kmax = max(kmax, sm.kmax[32 + lane]);
+  kmax = __reduce_max_sync(0xffffffffu, kmax);
+  // ---- the bin of the K-th largest key in a window of 16 binades below it, at 1/16 binade (bits
+  // 30..19 of the keys).  Every CTA sums the six faces' counts through distributed shared memory
+  // (6 KB; it moves ~6 B per cycle: a 2,048-bin histogram of all exponents, which needs no
+  // maximum, cost 8.5k cycles here), thread t the bin 255 - t.  The low half of a count is the
+  // map's, the high half that of the faces before this one (24,576 keys at most: no carry).
+  const int e_lo = (int)(kmax >> 23) - 15;
+  auto in_window = [&](uint32_t k) { return (int)(k >> 23) >= e_lo; };
+  auto bin_of = [&](uint32_t k) { return (((int)(k >> 23) - e_lo) << 4) | (int)((k >> 19) & 15u); };
+  if (owner)
+#pragma unroll
+    for (int u = 0; u < NK; ++u)
+      if (in_window(key[u])) atomicAdd(&sm.hist[bin_of(key[u])], 1u);
+  cluster.sync();
+  {
+    const int bin = 255 - tid;
+    uint32_t v[6], c = 0, all;
+#pragma unroll
+    for (int g = 0; g < 6; ++g) v[g] = cluster.map_shared_rank(sm.hist, g)[bin];
+#pragma unroll
+    for (int g = 0; g < 6; ++g) c += v[g] * (g < face ? 0x10001u : 1u);
+    const uint32_t incl = block_inclusive_sum(c & 0xFFFFu, sm.warp_tot, &all), start = incl - (c & 0xFFFFu);
+    sm.seg[bin] = start | (c << 16);
+    sm.cur[bin] = start + (c >> 16);
+    if (incl >= (uint32_t)K && start < (uint32_t)K) {
+      sm.scal[kScPrefix] = (int)((uint32_t)(((e_lo + (bin >> 4)) << 4) | (bin & 15)) << 19);
+      sm.scal[kScListed] = (int)incl;
+    }
+  }
+  __syncthreads();
+  const uint32_t lo_key = (uint32_t)sm.scal[kScPrefix];
+  const int n_list = sm.scal[kScListed];
+  if (n_list >= 0 && n_list <= list_cap(K)) {  // the same in all six CTAs
+    // ---- the keys of that bin and above are listed in every CTA, bin by bin from the top (within
+    // a bin by face), and each CTA ranks its own face's among their bin's; the first K are written
+    if (owner)
+#pragma unroll
+      for (int u = 0; u < NK; ++u)
+        if (key[u] >= lo_key) {
+          const int32_t gflat = face * SS + flat_of(u);
+          // composite key: larger key first, then smaller index first
+          const uint64_t ck = ((uint64_t)key[u] << 32) | (uint64_t)(0xFFFFFFFFu - (uint32_t)gflat);
+          const uint32_t slot = atomicAdd(&sm.cur[bin_of(key[u])], 1u);
+#pragma unroll
+          for (int g = 0; g < 6; ++g) cluster.map_shared_rank(sm.gkey, g)[slot] = ck;
+          if (u < NR) sm.gval[slot] = Winner{co[u < NR ? u : 0][0], co[u < NR ? u : 0][1], co[u < NR ? u : 0][2], gflat};
+          else sm.gval[slot] = Winner{ur, ug, ub, gflat};
+        }
+    cluster.sync();  // after it no CTA touches another's memory
+    for (int e = tid; e < n_list; e += kThreads) {
+      const uint64_t me = sm.gkey[e];
+      const int32_t gflat = (int32_t)(0xFFFFFFFFu - (uint32_t)me);
+      if (gflat / SS != face) continue;
+      const uint32_t sg = sm.seg[bin_of((uint32_t)(me >> 32))];
+      int rank = (int)(sg & 0xFFFFu);
+      const uint64_t* o = sm.gkey + rank;
+      const int n = (int)(sg >> 16);
+#pragma unroll 4
+      for (int i = 0; i < n; ++i) rank += o[i] > me;
+      if (rank < K) {
+        const Winner wv = sm.gval[e];
+        const size_t out = (size_t)env * K + rank;
+        idx_out[out] = wv.idx;
+        st_out[out * 3 + 0] = wv.r;
+        st_out[out * 3 + 1] = wv.g;
+        st_out[out * 3 + 2] = wv.b;
+      }
+    }
+    return;
+  }
+  cluster.sync();  // every CTA has read the histograms, whose memory the general form takes
+
+  // ---- too many keys in that bin (ties, all zeros) or too few in the window: 4-pass radix select of the K-th largest key
   uint32_t prefix = 0, mask = 0;
   int remaining = K;
   for (int pass = 0; pass < 4; ++pass) {
@@ -1042,9 +1144,12 @@ __global__ void __launch_bounds__(kThreads, 2)
   }
 }
 
-// Batches of at least this many maps use the batched kernel; smaller ones the cluster form,
-// whose six CTAs per map give the lower latency for a single map.
-constexpr int kBatchMinMaps = 32;
+// Batches of at least this many maps use the batched kernel; smaller ones the cluster form.  48
+// clusters of six run at once on 148 SMs, so 96 maps are two rounds of it; the batched kernel takes
+// the same time for 1 to 148 maps.  us at S = 64, K = 300 (K = 1024), cluster form and batched:
+// 32 maps 8.9 and 23.9 (13.3, 33.4), 64 maps 16.5 and 24.0 (24.6, 33.5), 98 maps 23.8 and 24.1
+// (35.0, 33.6), 147 maps 32.3 and 25.9 (48.0, 34.2).
+constexpr int kBatchMinMaps = 97;
 
 // A stream-ordered pool per device for the batched kernel's scratch.  It keeps its memory
 // between calls (release threshold = max), so a steady stream of batches allocates once.

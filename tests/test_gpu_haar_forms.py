@@ -1,0 +1,64 @@
+"""GPU tests of the two Haar + top-K forms on either side of the batch size that separates them
+(a cluster per map up to 96 maps, a persistent CTA per map from 97), bit for bit against the
+oracle, on maps that take each form's shortcuts and their fallbacks."""
+import numpy as np
+import pytest
+
+from neural_wavelet_prt_demo_b200 import synth
+from oracle import oracle as O
+from tests.helpers import bits_equal
+
+pytestmark = pytest.mark.gpu
+
+
+def _maps(S, K, E):
+    g = np.random.default_rng(S * 1000 + K)
+    f = np.stack([synth.make_env_faces(S, seed=7, index=e % 24) for e in range(E)])
+    f *= (1.0 + np.arange(E, dtype=np.float32) / 64).reshape(E, 1, 1, 1, 1)
+    h = max(1, S // 4)
+    edits = [
+        lambda m: m.__setitem__(slice(None), g.integers(0, 3, size=m.shape)),    # many equal keys
+        lambda m: m.__setitem__(slice(None), 1.0),                               # constant: all details 0
+        lambda m: m.__setitem__(slice(None), 0.0),                               # all keys 0
+        lambda m: m.__setitem__((1, 0, 0, 0), np.nan),
+        lambda m: m.__setitem__((4, S - 1, S - 1, 2), np.inf),
+        lambda m: m.__setitem__((2, slice(0, h), slice(0, h)), 1e4),             # winners in one corner
+        lambda m: m.__setitem__((0, 0, 0), 1e30),                                # range wider than any window
+        lambda m: m.__setitem__((5, S - 1, 0), 3e38),                            # overflow to inf on the way
+        lambda m: m.__imul__(-1.0),
+        lambda m: m.__imul__(1e-38),                                             # subnormal keys
+        lambda m: m.__imul__(np.float32(2.0) ** np.arange(-30, 30)[g.integers(0, 60, m.shape)]),  # wide range
+        lambda m: m.__setitem__(slice(1, 6), 0.0),                               # one face holds everything
+    ]
+    for i, edit in enumerate(edits):
+        if 2 * i + 1 < E:
+            edit(f[2 * i + 1])
+    return np.ascontiguousarray(f, np.float32)
+
+
+@pytest.mark.parametrize("S,K", [(64, 300), (64, 1), (64, 1024), (32, 64), (32, 1024), (16, 300), (8, 384), (4, 96),
+                                 (2, 24), (1, 6)])
+@pytest.mark.parametrize("E", [1, 25, 96, 97, 310])
+def test_haar_topk_forms_bit_exact(cuda, S, K, E):
+    import torch
+    from neural_wavelet_prt_demo_b200 import engine as eng
+    with np.errstate(all="ignore"):
+        f = _maps(S, K, E)
+    idx, st = eng.haar_topk(torch.from_numpy(f).to(cuda), K)
+    ridx, rst = O.haar_topk(f, K)
+    bad = np.nonzero((idx.cpu().numpy() != ridx).any(axis=1))[0]
+    assert bad.size == 0, bad[:10]
+    assert bits_equal(st.cpu().numpy(), rst)
+
+
+def test_haar_topk_unaligned_faces(cuda):
+    import torch
+    from neural_wavelet_prt_demo_b200 import engine as eng
+    for E in (1, 97):
+        f = _maps(64, 300, E)
+        buf = torch.empty(f.size + 1, dtype=torch.float32, device=cuda)
+        t = buf[1:].view(f.shape)
+        t.copy_(torch.from_numpy(f))
+        idx, st = eng.haar_topk(t, 300)
+        ridx, rst = O.haar_topk(f, 300)
+        assert np.array_equal(idx.cpu().numpy(), ridx) and bits_equal(st.cpu().numpy(), rst)
