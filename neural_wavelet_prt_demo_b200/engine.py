@@ -36,16 +36,26 @@ __all__ = ["RenderEngine", "EnvironmentMap", "FullFrame", "RenderConfig", "Nwprt
            "haar_topk", "env_rotate", "sh_project", "sh_dot"]
 
 
-def _ptr(t: Optional[torch.Tensor]):
-    return C.c_void_p(0 if t is None else t.data_ptr())
+# Pointers go to the library as plain ints (the bindings declare c_void_p arguments).  A wrapper
+# object per argument, a Stream object per call and an array's ctypes view cost more host time
+# than the launches of a short call: 13.3 us for a 4.5 us env_rotate, 18.5 us for haar_topk.
+
+def _ptr(t: Optional[torch.Tensor]) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
-def _stream_ptr(stream) -> C.c_void_p:
+# The current stream's handle without a Stream object around it (3.2 -> 0.3 us a call).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def _stream_ptr(stream) -> int:
     if stream is None:
-        return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        if _raw_stream is not None:
+            return _raw_stream(torch.cuda.current_device())
+        return torch.cuda.current_stream().cuda_stream
     if isinstance(stream, torch.cuda.Stream):
-        return C.c_void_p(stream.cuda_stream)
-    return C.c_void_p(int(stream))
+        return stream.cuda_stream
+    return int(stream)
 
 
 @dataclass
@@ -92,19 +102,21 @@ class FullFrame:
                          torch.zeros((n, 4), dtype=torch.float32, device=device))
 
     def gbuffer_struct(self) -> _lib.GBuffer:
-        for name in ("fbFirstHitPos", "fbworldNormal", "fbFirstHitReflecDir", "fbFirstHitKd",
-                     "fbFirstHitKs", "fbDirectDenoised"):
-            t = getattr(self, name)
-            if t.dtype != torch.float32 or not t.is_contiguous() or t.numel() != 4 * self.width * self.height:
+        n = self.width * self.height
+        float4 = (self.fbFirstHitPos, self.fbworldNormal, self.fbFirstHitReflecDir, self.fbFirstHitKd, self.fbFirstHitKs,
+                  self.fbDirectDenoised)
+        for i, t in enumerate(float4):
+            if t.dtype != torch.float32 or not t.is_contiguous() or t.numel() != 4 * n:
+                name = ("fbFirstHitPos", "fbworldNormal", "fbFirstHitReflecDir", "fbFirstHitKd", "fbFirstHitKs",
+                        "fbDirectDenoised")[i]
                 raise ValueError(f"{name} must be a contiguous float32 [N,4] tensor")
-        if self.fbRoughness.dtype != torch.float32 or self.fbRoughness.numel() != self.width * self.height:
+        if self.fbRoughness.dtype != torch.float32 or self.fbRoughness.numel() != n:
             raise ValueError("fbRoughness must be float32 [N]")
         if self.fbEnvironmentMapFlag.dtype not in (torch.uint8, torch.bool):
             raise ValueError("fbEnvironmentMapFlag must be uint8 or bool")
-        return _lib.GBuffer(self.width, self.height, *[
-            _ptr(getattr(self, n)) for n in ("fbFirstHitPos", "fbworldNormal", "fbFirstHitReflecDir",
-                                             "fbRoughness", "fbFirstHitKd", "fbFirstHitKs",
-                                             "fbDirectDenoised", "fbEnvironmentMapFlag")])
+        pos, nrm, refl, kd, ks, direct = (t.data_ptr() for t in float4)
+        return _lib.GBuffer(self.width, self.height, pos, nrm, refl, self.fbRoughness.data_ptr(), kd, ks, direct,
+                            self.fbEnvironmentMapFlag.data_ptr())
 
 
 def read_hdr(path: str) -> np.ndarray:
@@ -521,12 +533,12 @@ def haar_topk(faces: torch.Tensor, K: int, stream=None):
     if faces.dtype != torch.float32 or not faces.is_cuda or not faces.is_contiguous():
         raise ValueError("faces must be a contiguous float32 CUDA tensor")
     batched = faces.dim() == 5
-    f = faces if batched else faces.unsqueeze(0)
-    E, S = f.shape[0], f.shape[2]
-    idx = torch.empty((E, K), dtype=torch.int32, device=faces.device)
-    st = torch.empty((E, K, 3), dtype=torch.float32, device=faces.device)
-    check(lib().nwprt_haar_topk(_ptr(f), E, S, int(K), _ptr(idx), _ptr(st), _stream_ptr(stream)))
-    return (idx, st) if batched else (idx[0], st[0])
+    E, S = (faces.shape[0], faces.shape[2]) if batched else (1, faces.shape[1])
+    head = (E, K) if batched else (K,)
+    idx = torch.empty(head, dtype=torch.int32, device=faces.device)
+    st = torch.empty(head + (3,), dtype=torch.float32, device=faces.device)
+    check(lib().nwprt_haar_topk(faces.data_ptr(), E, S, int(K), idx.data_ptr(), st.data_ptr(), _stream_ptr(stream)))
+    return idx, st
 
 
 def tonemap_srgb(src: torch.Tensor, out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
@@ -550,7 +562,7 @@ def env_rotate(faces: torch.Tensor, R, out: Optional[torch.Tensor] = None, strea
     r = np.ascontiguousarray(np.asarray(R, np.float32).reshape(9))
     if out is None:
         out = torch.empty_like(faces)
-    check(lib().nwprt_env_rotate(_ptr(faces), faces.shape[1], r.ctypes.data_as(C.c_void_p), _ptr(out),
+    check(lib().nwprt_env_rotate(_ptr(faces), faces.shape[1], r.ctypes.data, _ptr(out),
                                  _stream_ptr(stream)))
     return out
 
