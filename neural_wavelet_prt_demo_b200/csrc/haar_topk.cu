@@ -1,5 +1,5 @@
 // Cubemap Haar transform + top-K wavelet selection: one thread-block cluster per env map for
-// single maps and small batches, one persistent CTA per map for batches of 97 maps or more
+// single maps and small batches, one persistent CTA per map for large batches
 // (haar_topk_batch_kernel, described where it is defined).
 //
 // The reference only loads precomputed results (waveletcoeffs/<name>.npy and
@@ -35,7 +35,7 @@
 // 25.0 -> 9.8 (radix select for all maps, all-pairs ranking, before).
 #include <cooperative_groups.h>
 
-#include <mutex>
+#include <type_traits>
 
 #include "nwprt_internal.cuh"
 
@@ -76,10 +76,7 @@ struct HaarSmem {
 // scal[] slots
 constexpr int kScPrefix = 0, kScMask = 1, kScRemaining = 2, kScCounter = 3, kScEq = 8;  // eq: [6]
 constexpr int kScListed = 14;                // cluster form: keys listed
-constexpr int kScNAbove = 16, kScNCand = 17;  // batched kernel: winners above the window bin, candidates in it
-// Candidates (keys in the window's selected bin) the batched kernel ranks directly; they share
-// the histogram region: composite keys (8 B) + ids (4 B).
-constexpr int kCandCap = 680;
+constexpr int kScNAbove = 16;                // batched kernel: keys in the final list
 
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
@@ -197,9 +194,9 @@ __device__ __forceinline__ void shuffle_level(float ll[3], int lane, int s, int 
   }
 }
 
-// shuffle_level with the details stored to a face's scratch slice, laid out [channel][thread]
+// shuffle_level with the details stored to the batched form's upper block, laid out [channel][thread]
 // (thread i * G + j owns upper-block entry (i, j)).
-__device__ __forceinline__ void shuffle_level_scratch(float ll[3], int lane, int s, int m, int h, bool live,
+__device__ __forceinline__ void shuffle_level_planar(float ll[3], int lane, int s, int m, int h, bool live,
                                                       float* upf, int G) {
   float v[3][3];
 #pragma unroll
@@ -231,6 +228,7 @@ struct FaceGeom {
   static constexpr int SS = S * S;
   static constexpr int NR = B == 4 ? 15 : (B == 2 ? 3 : 0);  // coefficients held in registers
   static constexpr int NK = NR + 1;                         // plus one entry of the upper block
+  static constexpr int FPI = T >= kThreads ? 1 : (kThreads / T < 6 ? kThreads / T : 6);  // faces a block holds at once
 };
 
 // Index within the face of thread tid's coefficient u (u == NR: its upper-block entry).
@@ -250,36 +248,33 @@ __device__ __forceinline__ int flat_in_face(int tid, int u) {
   return band == 0 ? i * S + j + h : (band == 1 ? (i + h) * S + j : (i + h) * S + j + h);
 }
 
-// Coefficient u < NR of thread tid's texel block (all three channels), recomputed from the
-// face at `src` with the same FP32 operations, in the same order, as the transform below:
-// a level-1 detail from its 2x2 quad, a level-2 detail from the four quads' LL values.  The
-// batched kernel keeps no copy of these coefficients; it recomputes the K winners' instead.
+// Channel c of coefficient u < NR of thread tid's texel block, recomputed from the face at `src`
+// with the same FP32 operations, in the same order, as the transform below: a level-1 detail from
+// its 2x2 quad, a level-2 detail from the four quads' LL values.  The batched kernel keeps no copy
+// of these coefficients; it recomputes the K winners' instead.
 template <int S>
-__device__ __forceinline__ void block_coef(const float* __restrict__ src, int tid, int u, float (&out)[3]) {
+__device__ __forceinline__ float block_coef(const float* __restrict__ src, int tid, int u, int c) {
   using F = FaceGeom<S>;
   const int bj = morton_even(tid), bi = morton_even(tid >> 1);
-  const float* blk = src + ((size_t)(F::B * bi) * S + F::B * bj) * 3;
+  const float* blk = src + ((size_t)(F::B * bi) * S + F::B * bj) * 3 + c;
   const int q = u / 3, band = u % 3;
-  auto quad = [&](int qi, int qj, int c, float& a, float& hl, float& lh, float& hh) {
-    const float* p0 = blk + ((size_t)(2 * qi) * S + 2 * qj) * 3 + c;
+  auto quad = [&](int qi, int qj, float& a, float& hl, float& lh, float& hh) {
+    const float* p0 = blk + ((size_t)(2 * qi) * S + 2 * qj) * 3;
     haar4(__ldg(p0), __ldg(p0 + 3), __ldg(p0 + S * 3), __ldg(p0 + S * 3 + 3), a, hl, lh, hh);
   };
+  float a, hl, lh, hh;
+  if (q < 4) {
+    quad(q >> 1, q & 1, a, hl, lh, hh);
+  } else {
+    float l1[4], x, y, z;
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    float a, hl, lh, hh;
-    if (q < 4) {
-      quad(q >> 1, q & 1, c, a, hl, lh, hh);
-    } else {
-      float l1[4], x, y, z;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) quad(k >> 1, k & 1, c, l1[k], x, y, z);
-      haar4(l1[0], l1[1], l1[2], l1[3], a, hl, lh, hh);
-    }
-    out[c] = band == 0 ? hl : (band == 1 ? lh : hh);
+    for (int k = 0; k < 4; ++k) quad(k >> 1, k & 1, l1[k], x, y, z);
+    haar4(l1[0], l1[1], l1[2], l1[3], a, hl, lh, hh);
   }
+  return band == 0 ? hl : (band == 1 ? lh : hh);
 }
 
-// The first part of the transform below, split out for the batched form: block_load loads
+// The first part of the transform below: block_load loads
 // thread t's B x B texel block (t < T), block_levels runs levels 1-2 on it in registers (co:
 // its NR detail coefficients, ll: the block's LL value), with the same operations in the same
 // order as haar_face_in_registers.
@@ -678,500 +673,606 @@ __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
 }
 
 // ------------------------------------------------------------------ batched form
-// One persistent CTA per map at a time (no cluster): for large batches, whole maps in flight
-// per SM beat the cluster's one sixth of a map each, and no step crosses an SM.  Faces are
-// transformed one after another with the same register code; the keys of all six stay in
-// shared memory (uint4 of four keys, thread-fastest: conflict-free).  Of the coefficients
-// only each thread's upper-block entry is kept, in this CTA's slice of a global scratch
-// buffer ([face][channel][thread], 18 KB at S = 64, so it stays in L2); the K winners' other
-// coefficients are recomputed from their texel blocks (block_coef), which costs far less
-// than writing and re-reading all 6 * S * S of them.  The select is block-local: a first
-// histogram pass over a window of 16 binades below the map's largest key; when that finds the
-// K-th largest key's bin, one scan sorts the keys above it (winners) from those in it
-// (candidates, ranked directly); otherwise radix passes, a bitmap of ties over the 6*S*S flat
-// indices and winner slots from one block scan.  The winners are ordered by a counting pass
-// over their key range.  The faces need no block barrier between them: levels 1-2 are
-// thread-local, levels 3-4 (warp shuffles) write their details straight to the scratch slice,
-// and the last levels of all six faces run after one barrier, in warps 0-5.
+// One persistent CTA per map at a time (no cluster): for large batches, whole maps in flight per
+// SM beat the cluster's one sixth of a map each, and no step crosses an SM.
+//
+// Few of a map's coefficients can be among its K largest, so their keys are not kept.  The CTA
+// transforms the six faces one after another, histogramming the first face's keys by their top 11
+// bits (the exponent and 3 bits of the fraction).  The K-th largest key seen so far is a lower bound
+// of the K-th largest of all: a warp lists only its keys from that one's bin up, counts what it
+// lists, and looks the bound up again at the third face, before it lists much of one (a face
+// brighter than the ones before), and from face to face once the list is crowded.
+// No barrier guards the look-up: counts still missing only lower the bound.  When the upper levels
+// are done, one block scan over the bins gives the last winner's bin, the listed keys from it up go
+// to their bin's part of a second list, and each is ranked among its own bin's keys only.  Keys
+// equal to 0 are never listed: a map with fewer than K others takes the first zeros by index.
+//
+// Levels 1-2 are thread-local; levels 3-4 (warp shuffles) leave their details in shared memory, and
+// the last levels of all six faces run after one barrier, in warps 0-5.  No other coefficient is
+// stored: the K winners' are recomputed from their texel blocks (block_coef).
+//
+// A map that overflows the first list goes over its keys once more; one whose last winner's bin is
+// too full (hundreds of equal keys) recomputes its keys in each pass of a radix select
+// (general_select).
+//
+// Small faces share the block: FPI of them are transformed at once.  Bound by latency and issue:
+// four CTAs of 64 registers fit an SM (1.09 us per map and SM slot), and what they leave of the
+// SM's memory as L1 matters, since a texel row's three 16-byte loads share their sectors (lists of
+// 6 K + 768 keys instead of 5 K + 512 took one step of it: 110 -> 117 us).  1,024 maps, K = 300:
+// 132 us -> 110 (2,790 GB/s) with all keys kept in shared memory, three scans of them and two CTAs
+// per SM before; K = 64 109 -> 88, K = 1024 229 -> 208; S = 32 102 -> 50; S = 16, K = 64 67 -> 19;
+// maps of few lights on black 269 -> 84.  Each face ten times brighter than the one before is the
+// bad case: 121 -> 174.
+
+constexpr int kBins = 2048;       // of keys by bits 30..20
+constexpr int kCtasPerSm = 4;
+
+__host__ __device__ constexpr int map_coeffs(int S) { return 6 * S * S; }
+// Keys that may be listed while the faces pass, and in the end.
+__host__ __device__ constexpr int face_list_cap(int S, int K) {
+  return 5 * K + 512 < map_coeffs(S) ? 5 * K + 512 : map_coeffs(S);
+}
 
 struct BatchSmem {
-  uint4* keys;      // [6][NK/4][kThreads]
-  uint32_t* whist;  // [kWarps][256] per-warp histograms of a pass
-  uint32_t* bits;   // [6*S*S/32] ties (aliases whist after the passes)
-  uint32_t* wpre;   // [6*S*S/32]
-  uint64_t* gkey;   // [K]
-  int* gid;         // [K] winner: (face * NK + u) * kThreads + thread
+  uint32_t* hist;   // [kBins + 1] counts (from the second scan on: where the bin's next key goes); then 0
+  uint32_t* lkey;   // [face_list_cap] keys listed while the faces pass
+  uint16_t* lid;    // [face_list_cap] their coefficient: (face * NK + u) * kThreads + thread
+  uint32_t* bits;   // [6*S*S/32] aliases lkey: listed (zero fill) or tied (general_select) indices
+  uint32_t* wpre;   // [6*S*S/32] exclusive popcount prefix of bits (general_select)
+  uint64_t* gkey;   // [list_cap] composite keys of the final list
+  uint16_t* gid;    // [list_cap]
+  uint16_t* order;  // [K] aliases lid: the winners' coefficients by rank
+  float* up;        // [6][3][kThreads] the upper-block entries: [face][channel][thread]
   float* llg;       // [6][16][3] each face's LL values left for its last levels
   int* warp_tot;
   int* scal;
 };
 
 __host__ __device__ inline size_t batch_smem_layout(int S, int K, char* base, BatchSmem* L) {
-  const int nk = S >= 4 ? 16 : (S == 2 ? 4 : 1);
-  const int nkq = (nk + 3) / 4;
-  const int nw = (6 * S * S + 31) / 32;
+  const int nw = (map_coeffs(S) + 31) / 32;
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o = align16(o + bytes); return at; };
-  const size_t oK = take(sizeof(uint4) * 6 * nkq * kThreads);
-  const size_t uA = sizeof(uint32_t) * kWarps * 256, uB = sizeof(uint32_t) * 2 * nw;
-  const size_t oH = take(uA > uB ? uA : uB);
-  const size_t oG = take(sizeof(uint64_t) * K);
-  const size_t oI = take(sizeof(int) * K);
-  const size_t oL = take(sizeof(float) * 3 * 16 * 6);
+  const size_t oH = take(sizeof(uint32_t) * (kBins + 4));
+  const size_t list = align16(sizeof(uint32_t) * face_list_cap(S, K)), both = sizeof(uint32_t) * 2 * nw;
+  const size_t oL = take(list > both ? list : both);
+  const size_t oI = take(sizeof(uint16_t) * face_list_cap(S, K));
+  const size_t oG = take(sizeof(uint64_t) * list_cap(K));
+  const size_t oD = take(sizeof(uint16_t) * list_cap(K));
+  const size_t oU = take(sizeof(float) * 6 * 3 * kThreads);
+  const size_t oLl = take(sizeof(float) * 3 * 16 * 6);
   const size_t oW = take(sizeof(int) * kWarps);
   const size_t oS = take(sizeof(int) * 32);
   if (L) {
-    L->keys = (uint4*)(base + oK);
-    L->whist = (uint32_t*)(base + oH);
-    L->bits = (uint32_t*)(base + oH);
-    L->wpre = (uint32_t*)(base + oH) + nw;
+    L->hist = (uint32_t*)(base + oH);
+    L->up = (float*)(base + oU);
+    L->order = (uint16_t*)(base + oI);
+    L->lkey = (uint32_t*)(base + oL);
+    L->bits = (uint32_t*)(base + oL);
+    L->wpre = (uint32_t*)(base + oL) + nw;
+    L->lid = (uint16_t*)(base + oI);
     L->gkey = (uint64_t*)(base + oG);
-    L->gid = (int*)(base + oI);
-    L->llg = (float*)(base + oL);
+    L->gid = (uint16_t*)(base + oD);
+    L->llg = (float*)(base + oLl);
     L->warp_tot = (int*)(base + oW);
     L->scal = (int*)(base + oS);
   }
   return o;
 }
 
+// The keys of the NR detail coefficients of texel block tid (0 for u == NR and for a thread without one)
+// and its block's LL value, with the operations of block_levels, two texel rows at a time.
 template <int S>
-__host__ __device__ constexpr size_t batch_scratch_floats_per_cta() {
-  return (size_t)6 * 3 * kThreads;
+__device__ __forceinline__ void face_keys(const float* __restrict__ src, bool owner, int tid,
+                                          uint32_t (&k)[FaceGeom<S>::NK], float (&ll)[3]) {
+  using F = FaceGeom<S>;
+  constexpr int B = F::B;
+#pragma unroll
+  for (int u = 0; u < F::NK; ++u) k[u] = 0u;
+  ll[0] = ll[1] = ll[2] = 0.f;
+  if (!owner) return;
+  const int bj = morton_even(tid), bi = morton_even(tid >> 1);
+  const float* blk = src + ((size_t)(B * bi) * S + B * bj) * 3;
+  if constexpr (B == 1) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) ll[c] = __ldg(blk + c);
+  } else {
+    float l1[B == 4 ? 4 : 1][3];
+    const bool vec = B == 4 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+#pragma unroll
+    for (int qi = 0; qi < B / 2; ++qi) {
+      float px[2][B * 3];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float* row = blk + (size_t)(2 * qi + r) * S * 3;
+        if (vec) {
+#pragma unroll
+          for (int q = 0; q < B * 3 / 4; ++q) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(row) + q);
+            px[r][4 * q] = v.x;
+            px[r][4 * q + 1] = v.y;
+            px[r][4 * q + 2] = v.z;
+            px[r][4 * q + 3] = v.w;
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < B * 3; ++q) px[r][q] = __ldg(row + q);
+        }
+      }
+#pragma unroll
+      for (int qj = 0; qj < B / 2; ++qj) {
+        const int q = qi * (B / 2) + qj;
+        float hl[3], lh[3], hh[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          haar4(px[0][6 * qj + c], px[0][6 * qj + 3 + c], px[1][6 * qj + c], px[1][6 * qj + 3 + c], l1[q][c], hl[c],
+                lh[c], hh[c]);
+        k[3 * q] = wavelet_key_bits(hl[0], hl[1], hl[2]);
+        k[3 * q + 1] = wavelet_key_bits(lh[0], lh[1], lh[2]);
+        k[3 * q + 2] = wavelet_key_bits(hh[0], hh[1], hh[2]);
+      }
+    }
+    if constexpr (B == 4) {
+      float hl[3], lh[3], hh[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) haar4(l1[0][c], l1[1][c], l1[2][c], l1[3][c], ll[c], hl[c], lh[c], hh[c]);
+      k[12] = wavelet_key_bits(hl[0], hl[1], hl[2]);
+      k[13] = wavelet_key_bits(lh[0], lh[1], lh[2]);
+      k[14] = wavelet_key_bits(hh[0], hh[1], hh[2]);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) ll[c] = l1[0][c];
+    }
+  }
+}
+
+// The coefficient ((face * NK + u) * kThreads + thread) at flat index g of the map: flat_in_face
+// turned around.
+template <int S>
+__device__ __forceinline__ int id_of_flat(int g) {
+  using F = FaceGeom<S>;
+  constexpr int G = F::G;
+  const int f = g / F::SS, i = (g % F::SS) / S, j = g % S;
+  int t, u;
+  if (i < G && j < G) {
+    t = i * G + j;
+    u = F::NR;
+  } else {
+    const bool second = F::B == 4 && i < S / 2 && j < S / 2;  // level 2, else level 1
+    const int h = second ? S / 4 : S / 2;
+    const int band = i < h ? 0 : (j < h ? 1 : 2), ii = i < h ? i : i - h, jj = j < h ? j : j - h;
+    const int bi = F::B == 4 && !second ? ii / 2 : ii, bj = F::B == 4 && !second ? jj / 2 : jj;
+    const int q = F::B == 4 ? (second ? 4 : (ii & 1) * 2 + (jj & 1)) : 0;
+    t = 0;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) t |= ((bj >> b & 1) << (2 * b)) | ((bi >> b & 1) << (2 * b + 1));
+    u = 3 * q + band;
+  }
+  return (f * F::NK + u) * kThreads + t;
+}
+
+// Lower edge of the bin that holds the K-th largest key counted so far (0: fewer than K), by one
+// warp: 64 bins a lane from the top, then the crossing lane's bins two a lane.
+__device__ __forceinline__ uint32_t kth_bin_edge(const uint32_t* hist, int K, int lane) {
+  const uint32_t h = smem_u32(hist + kBins - 64 * (lane + 1));
+  uint32_t sum = 0;
+#pragma unroll 4
+  for (int i = 0; i < 16; ++i) {
+    uint4 v;  // lanes on different banks
+    asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(h + ((i + lane) & 15) * 16)
+                 : "memory");
+    sum += v.x + v.y + v.z + v.w;
+  }
+  uint32_t incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  const uint32_t hit = __ballot_sync(0xffffffffu, incl >= (uint32_t)K);
+  if (!hit) return 0u;
+  const int l = __ffs(hit) - 1;
+  const uint32_t before = __shfl_sync(0xffffffffu, incl - sum, l);
+  const int top = kBins - 64 * l - 1;
+  const volatile uint32_t* hv = hist;
+  const uint32_t a = hv[top - 2 * lane], b = hv[top - 2 * lane - 1];
+  uint32_t in2 = a + b;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, in2, o);
+    if (lane >= o) in2 += t;
+  }
+  const uint32_t hit2 = __ballot_sync(0xffffffffu, before + in2 >= (uint32_t)K);
+  if (!hit2) return (uint32_t)(top - 63) << 20;  // counts only grow: the bin is one of these 64
+  const int l2 = __ffs(hit2) - 1;
+  const bool in_b = __shfl_sync(0xffffffffu, before + in2 - b < (uint32_t)K, l2);
+  return (uint32_t)(top - 2 * l2 - (in_b ? 1 : 0)) << 20;
+}
+
+// What a warp lists of the keys it forms (see above).
+struct KeyList {
+  const BatchSmem& sm;
+  int K, cap, lane;
+  uint32_t bound = 1u;   // keys of 0 are neither counted nor listed
+  bool crowded = false;  // the list fills faster than faces alike would fill it
+
+  __device__ __forceinline__ void raise() { bound = max(bound, kth_bin_edge(sm.hist, K, lane)); }
+
+  // Lists the warp's keys k[0..N) from the bound up, and counts them unless they have been; id(u):
+  // coefficient of this lane's k[u].
+  template <int N, class ID>
+  __device__ __forceinline__ void add(const uint32_t (&k)[N], int n_keys, bool counted, const ID& id) {
+    uint32_t hits = 0;  // by u
+    auto compare = [&] {
+      hits = 0;
+#pragma unroll
+      for (int u = 0; u < N; ++u)
+        if (u < n_keys) hits |= k[u] >= bound ? 1u << u : 0u;
+      return (int)__reduce_add_sync(0xffffffffu, (uint32_t)__popc(hits));
+    };
+    int total = compare();
+    if (!counted && total > max(32, K * 3 / 16)) {  // a brighter face: raise the bound before it is listed
+#pragma unroll
+      for (int u = 0; u < N; ++u)
+        if (hits >> u & 1u) atomicAdd(&sm.hist[k[u] >> 20], 1u);
+      __syncwarp();
+      raise();
+      total = compare();
+      counted = true;
+    }
+    if (total == 0) return;
+    int at = 0;
+    if (lane == 0) at = atomicAdd(&sm.scal[kScListed], total);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    crowded |= at > 4 * K + 384;
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      const bool h = hits >> u & 1u;
+      const uint32_t b = __ballot_sync(0xffffffffu, h);
+      const int p = at + __popc(b & ((1u << lane) - 1u));
+      if (h && p < cap) {
+        sm.lkey[p] = k[u];
+        sm.lid[p] = (uint16_t)id(u);
+      }
+      if (h && !counted) atomicAdd(&sm.hist[k[u] >> 20], 1u);  // also past the list's end
+      at += __popc(b);
+    }
+  }
+};
+
+// Lists a map's keys once more, those from lo_key up (counts untouched).
+template <int S>
+__device__ __noinline__ void list_again(const float* __restrict__ map, uint32_t lo_key, int K) {
+  using F = FaceGeom<S>;
+  extern __shared__ __align__(16) char smem_raw[];
+  BatchSmem sm;
+  batch_smem_layout(S, K, smem_raw, &sm);
+  const int tid = threadIdx.x, cap = face_list_cap(S, K);
+  KeyList list{sm, K, cap, tid & 31};
+  list.bound = lo_key;
+  const int lt = tid % F::T, fi = tid / F::T;
+  __syncthreads();
+  if (tid == 0) sm.scal[kScListed] = 0;
+  __syncthreads();
+#pragma unroll 1
+  for (int f0 = 0; f0 < 6; f0 += F::FPI) {
+    const int f = f0 + fi;
+    const bool owner = fi < F::FPI && f < 6;
+    uint32_t k[F::NK];
+    float ll[3];
+    face_keys<S>(map + (size_t)f * F::SS * 3, owner, lt, k, ll);
+    const float* upf = sm.up + f * 3 * kThreads;
+    if (owner) k[F::NR] = wavelet_key_bits(upf[lt], upf[kThreads + lt], upf[2 * kThreads + lt]);
+    list.add(k, F::NK, true, [&](int u) { return (f * F::NK + u) * kThreads + lt; });
+  }
+  __syncthreads();
+}
+
+// The K winners of a map whose lists overflowed, into gkey / gid: a 4-pass 8-bit radix select that
+// recomputes the keys in each pass, then ties at the threshold in flat-index order by a bitmap.
+template <int S>
+__device__ __noinline__ void general_select(const float* __restrict__ map, int K) {
+  using F = FaceGeom<S>;
+  extern __shared__ __align__(16) char smem_raw[];
+  BatchSmem sm;
+  batch_smem_layout(S, K, smem_raw, &sm);
+  const float* up = sm.up;
+  constexpr int SS = F::SS, NR = F::NR, NK = F::NK, NW = (6 * SS + 31) / 32;
+  const int tid = threadIdx.x, lt = tid % F::T, fi = tid / F::T;
+  uint32_t prefix = 0, mask = 0, thr = 0;
+  int remaining = K, n_sel = 0, slot = 0;
+  __syncthreads();
+  for (int w = tid; w < NW; w += kThreads) sm.bits[w] = 0u;
+  // passes 0-3: the threshold; 4: the ties' bitmap; 5: each thread's winners; 6: their slots
+  for (int pass = 0; pass < 7; ++pass) {
+    const int shift = 24 - 8 * pass;
+    if (pass < 4) sm.hist[tid] = 0u;
+    __syncthreads();
+    if (pass == 5) {
+      constexpr int PER = (NW + kThreads - 1) / kThreads;
+      uint32_t mine = 0, all;
+      for (int i = 0; i < PER; ++i) mine += tid * PER + i < NW ? (uint32_t)__popc(sm.bits[tid * PER + i]) : 0u;
+      uint32_t run = block_inclusive_sum(mine, sm.warp_tot, &all) - mine;
+      for (int i = 0; i < PER; ++i)
+        if (tid * PER + i < NW) {
+          sm.wpre[tid * PER + i] = run;
+          run += (uint32_t)__popc(sm.bits[tid * PER + i]);
+        }
+      __syncthreads();
+    }
+    if (pass == 6) {
+      uint32_t all;
+      slot = (int)block_inclusive_sum((uint32_t)n_sel, sm.warp_tot, &all) - n_sel;
+    }
+    for (int f = fi; f < 6 && fi < F::FPI; f += F::FPI) {
+      uint32_t k[NK];
+      float ll[3];
+      face_keys<S>(map + (size_t)f * SS * 3, true, lt, k, ll);
+      const float* upf = up + f * 3 * kThreads;
+      k[NR] = wavelet_key_bits(upf[lt], upf[kThreads + lt], upf[2 * kThreads + lt]);
+#pragma unroll
+      for (int u = 0; u < NK; ++u) {
+        if (pass < 4) {
+          if ((k[u] & mask) == prefix) atomicAdd(&sm.hist[(k[u] >> shift) & 255u], 1u);
+          continue;
+        }
+        if (k[u] < thr) continue;
+        const int g = f * SS + flat_in_face<S>(lt, u), w = g >> 5;
+        if (pass == 4) {
+          if (k[u] == thr) atomicOr(&sm.bits[w], 1u << (g & 31));
+          continue;
+        }
+        if (k[u] == thr && (int)(sm.wpre[w] + __popc(sm.bits[w] & ((1u << (g & 31)) - 1u))) >= remaining) continue;
+        if (pass == 5) {
+          ++n_sel;
+        } else {
+          sm.gkey[slot] = ((uint64_t)k[u] << 32) | (uint64_t)(0xFFFFFFFFu - (uint32_t)g);
+          sm.gid[slot] = (uint16_t)((f * NK + u) * kThreads + lt);
+          ++slot;
+        }
+      }
+    }
+    __syncthreads();
+    if (pass < 4) {
+      const int digit = 255 - tid;
+      uint32_t all;
+      const uint32_t tot = sm.hist[digit];
+      const uint32_t incl = block_inclusive_sum(tot, sm.warp_tot, &all);
+      if (incl >= (uint32_t)remaining && incl - tot < (uint32_t)remaining) {
+        sm.scal[kScPrefix] = (int)(prefix | ((uint32_t)digit << shift));
+        sm.scal[kScRemaining] = remaining - (int)(incl - tot);
+      }
+      __syncthreads();
+      prefix = (uint32_t)sm.scal[kScPrefix];
+      remaining = sm.scal[kScRemaining];
+      mask |= 255u << shift;
+      thr = prefix;
+    }
+  }
 }
 
 template <int S>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, kCtasPerSm)
     haar_topk_batch_kernel(const float* __restrict__ faces, int n_env, int K, int32_t* __restrict__ idx_out,
-                           float* __restrict__ st_out, float* __restrict__ scratch) {
+                           float* __restrict__ st_out) {
   using F = FaceGeom<S>;
-  constexpr int T = F::T, SS = F::SS, NR = F::NR, NK = F::NK;
-  constexpr int NKQ = (NK + 3) / 4;
-  constexpr int NW = (6 * SS + 31) / 32;
+  constexpr int T = F::T, SS = F::SS, NR = F::NR, NK = F::NK, G = F::G;
+  constexpr int NL = G >= 8 ? G / 4 : 1;  // side of the LL grid left after levels 3-4
   static_assert(T <= kThreads, "one 4x4 block per thread");
-  static_assert(kThreads == 256, "one thread per bin of the winners' counting pass");
-  static_assert(512 * sizeof(uint32_t) + kMaxK * sizeof(uint16_t) <= kWarps * 256 * sizeof(uint32_t),
-                "the winners' bins and order fit the histogram region");
+  static_assert(6 * NK * kThreads <= 65536, "coefficient ids are 16-bit");
   extern __shared__ __align__(16) char smem_raw[];
   BatchSmem sm;
   batch_smem_layout(S, K, smem_raw, &sm);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const bool owner = tid < T;
-  // this CTA's upper-block entries, [face][channel][thread]
-  float* up = scratch + (size_t)blockIdx.x * batch_scratch_floats_per_cta<S>();
+  const int lt = tid % T, fi = tid / T;  // texel block, and which of the FPI faces at a time
+  const int cap = face_list_cap(S, K);
+  float* up = sm.up;
+  int* n_listed = &sm.scal[kScListed];
 
   for (int env = blockIdx.x; env < n_env; env += gridDim.x) {
-    // ---- the six transforms, with no block barrier between faces: levels 1-2 in registers
-    // (their 15 keys straight to shared memory), levels 3-4 by warp shuffles whose details go
-    // to this face's scratch slice, the LL values left over to shared staging.  After all six,
-    // warp f finishes face f's last levels; then every thread reads its own six upper-block
-    // entries and forms their keys.  Each thread keeps the largest key it formed.
-    uint32_t kmax = 0;
-    constexpr int G = F::G;
-    constexpr int NL = G >= 8 ? G / 4 : 1;  // side of the LL grid left after levels 3-4
-    for (int f = 0; f < 6; ++f) {
-      const float* src = faces + ((size_t)env * 6 + f) * (size_t)SS * 3;
-      // the next face (after the sixth: this CTA's next map's first) into L2 meanwhile
+    const float* map = faces + (size_t)env * 6 * SS * 3;
+    for (int i = tid; i < kBins / 4; i += kThreads) reinterpret_cast<uint4*>(sm.hist)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (tid == 0) *n_listed = 0;
+    __syncthreads();
+    KeyList list{sm, K, cap, lane};
+    for (int f0 = 0; f0 < 6; f0 += F::FPI) {
+      const int f = f0 + fi;
+      const bool owner = fi < F::FPI && f < 6;
+      // the next faces (after the last: this CTA's next map's first) into L2 meanwhile
       if (tid == 0 && (SS * 12) % 16 == 0) {
-        const long long nxt = (long long)env * 6 + f + 1 + (f == 5 ? (long long)(gridDim.x - 1) * 6 : 0);
+        const int n_pf = f0 + F::FPI >= 6 ? F::FPI : min(F::FPI, 6 - f0 - F::FPI);
+        const long long nxt = f0 + F::FPI >= 6 ? (long long)(env + gridDim.x) * 6 : (long long)env * 6 + f0 + F::FPI;
         const float* pf = faces + (size_t)nxt * SS * 3;
         if (nxt < (long long)n_env * 6 && (reinterpret_cast<uintptr_t>(pf) & 15) == 0)
-          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(pf), "r"((uint32_t)(SS * 12)) : "memory");
+          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(pf), "r"((uint32_t)(n_pf * SS * 12)) : "memory");
       }
       float* upf = up + f * 3 * kThreads;
-      uint32_t k[NKQ * 4];
-#pragma unroll
-      for (int u = 0; u < NKQ * 4; ++u) k[u] = 0u;
+      uint32_t k[NK];
       float ll[3];
+      face_keys<S>(map + (size_t)f * SS * 3, owner, lt, k, ll);
+      if (f0 == 0) {
+#pragma unroll
+        for (int u = 0; u < NR; ++u)
+          if (k[u]) atomicAdd(&sm.hist[k[u] >> 20], 1u);
+      }
       {
-        float px[F::B][F::B][3];
-        float co[NR > 0 ? NR : 1][3];
-        block_load<S>(src, tid, px);
-        block_levels<S>(px, tid, co, ll);
-        if (owner)
-#pragma unroll
-          for (int u = 0; u < NR; ++u) {
-            k[u] = wavelet_key_bits(co[u][0], co[u][1], co[u][2]);
-            kmax = max(kmax, k[u]);
-          }
-      }
-#pragma unroll
-      for (int q = 0; q < NKQ; ++q)
-        sm.keys[((size_t)f * NKQ + q) * kThreads + tid] = make_uint4(k[4 * q], k[4 * q + 1], k[4 * q + 2], k[4 * q + 3]);
-      int n = G, st_ = 1;
-#pragma unroll
-      for (int lev = 0; lev < 2; ++lev)
-        if (n >= 2) {
-          shuffle_level_scratch(ll, lane, st_, tid / (4 * st_), n / 2, owner, upf, G);
-          n /= 2;
-          st_ *= 4;
-        }
-      if (n >= 2) {
-        if (owner && (tid & (st_ - 1)) == 0)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) sm.llg[(f * 16 + tid / st_) * 3 + c] = ll[c];
-      } else if (tid == 0) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) upf[c * kThreads] = ll[c];  // the DC term
-      }
-    }
-    __syncthreads();  // every face's level-3/4 details and LL staging are written
-    if constexpr (NL >= 2) {
-      if (warp < 6) {
-        const int f = warp;
-        float* upf = up + f * 3 * kThreads;
-        const bool live = lane < NL * NL;
-        float ll[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) ll[c] = live ? sm.llg[(f * 16 + lane) * 3 + c] : 0.f;
-        int n = NL, s2 = 1;
+        int n = G, st = 1;
 #pragma unroll
         for (int lev = 0; lev < 2; ++lev)
           if (n >= 2) {
-            shuffle_level_scratch(ll, lane, s2, lane / (4 * s2), n / 2, live, upf, G);
+            shuffle_level_planar(ll, lane, st, lt / (4 * st), n / 2, owner, upf, G);
             n /= 2;
-            s2 *= 4;
+            st *= 4;
           }
-        if (lane == 0)
+        if (n >= 2) {
+          if (owner && (lt & (st - 1)) == 0)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) sm.llg[(f * 16 + lt / st) * 3 + c] = ll[c];
+        } else if (owner && lt == 0) {
 #pragma unroll
           for (int c = 0; c < 3; ++c) upf[c * kThreads] = ll[c];  // the DC term
+        }
+        if (f0 == 0) __syncthreads();  // the first faces' counts: without them no bound
+        if (NR > 0 && (f0 == 0 || f0 == 2 || list.crowded)) list.raise();
       }
-      __syncthreads();  // the last levels' details are written
+      if constexpr (NR > 0) {
+        list.add(k, NR, f0 == 0, [&](int u) { return (f * NK + u) * kThreads + lt; });
+      }
     }
-    if (owner)
-      for (int f = 0; f < 6; ++f) {
+    {
+      __syncthreads();  // every face's level-3/4 details and LL staging are written
+      if constexpr (NL >= 2) {
+        if (warp < 6) {
+          const int f = warp;
+          float* upf = up + f * 3 * kThreads;
+          const bool live = lane < NL * NL;
+          float ll[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) ll[c] = live ? sm.llg[(f * 16 + lane) * 3 + c] : 0.f;
+          int n = NL, s2 = 1;
+#pragma unroll
+          for (int lev = 0; lev < 2; ++lev)
+            if (n >= 2) {
+              shuffle_level_planar(ll, lane, s2, lane / (4 * s2), n / 2, live, upf, G);
+              n /= 2;
+              s2 *= 4;
+            }
+          if (lane == 0)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) upf[c * kThreads] = ll[c];  // the DC term
+        }
+        __syncthreads();  // the last levels' details are written
+      }
+    }
+    {
+      constexpr int NF = (6 + F::FPI - 1) / F::FPI;
+      uint32_t k[NF];
+#pragma unroll
+      for (int i = 0; i < NF; ++i) {
+        const int f = i * F::FPI + fi;
         const float* upf = up + f * 3 * kThreads;
-        const uint32_t kk = wavelet_key_bits(upf[tid], upf[kThreads + tid], upf[2 * kThreads + tid]);
-        kmax = max(kmax, kk);
-        reinterpret_cast<uint32_t*>(&sm.keys[((size_t)f * NKQ + NR / 4) * kThreads + tid])[NR % 4] = kk;
+        const bool owner = fi < F::FPI && f < 6;
+        k[i] = owner ? wavelet_key_bits(upf[lt], upf[kThreads + lt], upf[2 * kThreads + lt]) : 0u;
       }
-    __syncthreads();  // the keys are complete
-    // ---- radix select of the K-th largest key.  The keys' top bits are mostly exponent, so a
-    // plain first pass piles 24K keys into a few bins (serialised shared atomics).  Instead the
-    // first pass histograms only keys within 16 binades of the largest key, at 1/16 binade
-    // (256 bins on bits 30..19; keys are non-negative, bit 31 is 0).  If that window holds K
-    // keys or more, the K-th largest is in it and the remaining 19 bits take passes of 8, 8
-    // and 3 bits over the few keys that match the prefix; otherwise four 8-bit passes.
-    uint32_t prefix = 0, mask = 0;
-    int remaining = K;
-    int shifts[4] = {24, 16, 8, 0}, widths[4] = {8, 8, 8, 8}, n_pass = 4;
+      list.add(k, NF, false, [&](int i) { return ((i * F::FPI + fi) * NK + NR) * kThreads + lt; });
+    }
+    if (tid == 0) {
+      sm.scal[kScPrefix] = 1;  // every listed key, if they are fewer than K
+      sm.scal[kScNAbove] = -1;
+    }
+    __syncthreads();
+    // ---- the last winner's bin: eight bins a thread from the top.  A bin's part of the final list
+    // starts after the keys of all bins above it.
     {
-      kmax = __reduce_max_sync(0xffffffffu, kmax);  // then over the block: the map's largest key
-      if (lane == 0) sm.warp_tot[warp] = (int)kmax;
-      for (int i = tid; i < kWarps * 256; i += kThreads) sm.whist[i] = 0u;
-      __syncthreads();
+      const int b0 = kBins - 8 - 8 * tid;
+      uint4* h4 = reinterpret_cast<uint4*>(sm.hist + b0);
+      const uint4 lo4 = h4[0], hi4 = h4[1];
+      const uint32_t c[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
+      uint32_t sum = 0, all, start[8];
 #pragma unroll
-      for (int w = 0; w < kWarps; ++w) kmax = max(kmax, (uint32_t)sm.warp_tot[w]);
-      const int e_lo = (int)(kmax >> 23) - 15;
-      if (owner) {
-        uint32_t* h = sm.whist + warp * 256;
-        for (int f = 0; f < 6; ++f)
+      for (int i = 0; i < 8; ++i) sum += c[i];
+      const uint32_t incl = block_inclusive_sum(sum, sm.warp_tot, &all);
+      uint32_t run = incl - sum;
 #pragma unroll
-          for (int q = 0; q < NKQ; ++q) {
-            const uint4 v = sm.keys[((size_t)f * NKQ + q) * kThreads + tid];
-            const uint32_t kk[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int e = (int)(kk[i] >> 23);
-              if (4 * q + i < NK && e >= e_lo) atomicAdd(&h[((e - e_lo) << 4) | ((kk[i] >> 19) & 15u)], 1u);
-            }
-          }
-      }
-      __syncthreads();
-      const int bin = 255 - tid;
-      uint32_t tot = 0;
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) tot += sm.whist[w * 256 + bin];
-      uint32_t all;
-      const uint32_t incl = block_inclusive_sum(tot, sm.warp_tot, &all);  // its barriers order the reads above
-      if (tid == 0) sm.scal[kScRemaining] = -1;  // stays -1 when the window holds fewer than K keys
-      __syncthreads();
-      if (incl >= (uint32_t)K && incl - tot < (uint32_t)K) {
-        sm.scal[kScPrefix] = (int)((uint32_t)(((e_lo + (bin >> 4)) << 4) | (bin & 15)) << 19);
-        sm.scal[kScRemaining] = K - (int)(incl - tot);
-      }
-      __syncthreads();
-      if (sm.scal[kScRemaining] >= 0) {
-        prefix = (uint32_t)sm.scal[kScPrefix];
-        mask = 0xFFF80000u;
-        remaining = sm.scal[kScRemaining];
-        shifts[0] = 11;
-        shifts[1] = 3;
-        shifts[2] = 0;
-        widths[2] = 3;
-        n_pass = 3;
-      }
-    }
-    // ---- the window's bin was found: every key above it wins, the keys in it are candidates.
-    // Two scans sort them without atomics: the first counts each thread's keys above the bin
-    // and in it, one block scan of both counts (packed in one word; each total is below 2^16)
-    // gives every thread its slots, and the second writes them.  A group of four keys below
-    // the bin (almost all of them) costs one compare per scan.  The candidates, usually a few
-    // dozen, are ranked among themselves.  More candidates than fit: the general passes below.
-    bool fast = false;
-    if (n_pass == 3) {
-      uint64_t* ckey = reinterpret_cast<uint64_t*>(sm.whist);
-      int* cid = reinterpret_cast<int*>(ckey + kCandCap);
-      const uint32_t lo_key = prefix, hi_key = prefix + (1u << 19);  // the bin is [lo_key, hi_key)
-      uint32_t n_up = 0, n_in = 0;
-      if (owner)
-        for (int f = 0; f < 6; ++f)
-#pragma unroll
-          for (int q = 0; q < NKQ; ++q) {
-            const uint4 v = sm.keys[((size_t)f * NKQ + q) * kThreads + tid];
-            if (max(max(v.x, v.y), max(v.z, v.w)) < lo_key) continue;
-            const uint32_t kk[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const bool live = 4 * q + i < NK;
-              n_up += live && kk[i] >= hi_key;
-              n_in += live && kk[i] >= lo_key && kk[i] < hi_key;
-            }
-          }
-      uint32_t all;
-      const uint32_t packed = n_up | (n_in << 16);
-      const uint32_t excl = block_inclusive_sum(packed, sm.warp_tot, &all) - packed;  // barriers inside
-      uint32_t slot_up = excl & 0xFFFFu, slot_in = excl >> 16;
-      if (owner && packed)
-        for (int f = 0; f < 6; ++f)
-#pragma unroll
-          for (int q = 0; q < NKQ; ++q) {
-            const uint4 v = sm.keys[((size_t)f * NKQ + q) * kThreads + tid];
-            if (max(max(v.x, v.y), max(v.z, v.w)) < lo_key) continue;
-            const uint32_t kk[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int u = 4 * q + i;
-              if (u >= NK || kk[i] < lo_key) continue;
-              const int g = f * SS + flat_in_face<S>(tid, u);
-              const uint64_t ck = ((uint64_t)kk[i] << 32) | (uint64_t)(0xFFFFFFFFu - (uint32_t)g);
-              const int id = (f * NK + u) * kThreads + tid;
-              if (kk[i] >= hi_key) {
-                sm.gkey[slot_up] = ck;
-                sm.gid[slot_up] = id;
-                ++slot_up;
-              } else {
-                if (slot_in < (uint32_t)kCandCap) {
-                  ckey[slot_in] = ck;
-                  cid[slot_in] = id;
-                }
-                ++slot_in;
-              }
-            }
-          }
-      if (tid == 0) {
-        sm.scal[kScNAbove] = (int)(all & 0xFFFFu);
-        sm.scal[kScNCand] = (int)(all >> 16);
-      }
-      __syncthreads();
-      const int n_cand = sm.scal[kScNCand];
-      if (n_cand <= kCandCap) {
-        fast = true;
-        const int n_above = sm.scal[kScNAbove];  // == K - remaining
-        for (int c = tid; c < n_cand; c += kThreads) {
-          const uint64_t me = ckey[c];
-          int rank = 0;
-          for (int o = 0; o < n_cand; ++o) rank += ckey[o] > me;
-          if (rank < remaining) {
-            sm.gkey[n_above + rank] = me;
-            sm.gid[n_above + rank] = cid[c];
-          }
+      for (int i = 7; i >= 0; --i) {
+        start[i] = run;
+        if (run < (uint32_t)K && run + c[i] >= (uint32_t)K) {
+          sm.scal[kScPrefix] = max(1, (b0 + i) << 20);
+          sm.scal[kScNAbove] = (int)(run + c[i]);
         }
-        __syncthreads();
+        run += c[i];
       }
-    }
-    if (!fast) {
-      for (int pass = 0; pass < n_pass; ++pass) {
-        const int shift = shifts[pass];
-        const uint32_t dmask = (1u << widths[pass]) - 1u;
-        for (int i = tid; i < kWarps * 256; i += kThreads) sm.whist[i] = 0u;
-        __syncthreads();
-        if (owner) {
-          uint32_t* h = sm.whist + warp * 256;
-          for (int f = 0; f < 6; ++f)
-  #pragma unroll
-            for (int q = 0; q < NKQ; ++q) {
-              const uint4 v = sm.keys[((size_t)f * NKQ + q) * kThreads + tid];
-              const uint32_t kk[4] = {v.x, v.y, v.z, v.w};
-  #pragma unroll
-              for (int i = 0; i < 4; ++i)
-                if (4 * q + i < NK && (kk[i] & mask) == prefix) atomicAdd(&h[(kk[i] >> shift) & dmask], 1u);
-            }
-        }
-        __syncthreads();
-        const int digit = 255 - tid;  // digits above dmask hold no keys
-        uint32_t tot = 0;
-  #pragma unroll
-        for (int w = 0; w < kWarps; ++w) tot += sm.whist[w * 256 + digit];
-        uint32_t all;
-        const uint32_t incl = block_inclusive_sum(tot, sm.warp_tot, &all);
-        if (incl >= (uint32_t)remaining && incl - tot < (uint32_t)remaining) {
-          sm.scal[kScPrefix] = (int)(prefix | ((uint32_t)digit << shift));
-          sm.scal[kScMask] = (int)(mask | (dmask << shift));
-          sm.scal[kScRemaining] = remaining - (int)(incl - tot);
-        }
-        __syncthreads();
-        prefix = (uint32_t)sm.scal[kScPrefix];
-        mask = (uint32_t)sm.scal[kScMask];
-        remaining = sm.scal[kScRemaining];
-      }
-      // ---- ties at the threshold in flat-index order: a bitmap over face * S*S + flat
-      const uint32_t thr = prefix;
-      for (int w = tid; w < NW; w += kThreads) sm.bits[w] = 0u;
-      __syncthreads();
-      if (owner)
-        for (int f = 0; f < 6; ++f)
-  #pragma unroll
-          for (int q = 0; q < NKQ; ++q) {
-            const uint4 v = sm.keys[((size_t)f * NKQ + q) * kThreads + tid];
-            const uint32_t kk[4] = {v.x, v.y, v.z, v.w};
-  #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              if (4 * q + i < NK && kk[i] == thr) {
-                const int g = f * SS + flat_in_face<S>(tid, 4 * q + i);
-                atomicOr(&sm.bits[g >> 5], 1u << (g & 31));
-              }
-          }
-      __syncthreads();
-      {
-        // exclusive popcount prefix over the bitmap: thread t covers words [t*per, t*per + per)
-        constexpr int PER = (NW + kThreads - 1) / kThreads;
-        uint32_t pc[PER], mine = 0;
-  #pragma unroll
-        for (int i = 0; i < PER; ++i) {
-          const int w = tid * PER + i;
-          pc[i] = w < NW ? (uint32_t)__popc(sm.bits[w]) : 0u;
-          mine += pc[i];
-        }
-        uint32_t all;
-        uint32_t run = block_inclusive_sum(mine, sm.warp_tot, &all) - mine;
-  #pragma unroll
-        for (int i = 0; i < PER; ++i) {
-          const int w = tid * PER + i;
-          if (w < NW) sm.wpre[w] = run;
-          run += pc[i];
-        }
-      }
-      __syncthreads();
-      // ---- winners: slots from one block scan of per-thread counts
-      int n_sel = 0;
-      if (owner)
-        for (int f = 0; f < 6; ++f)
-  #pragma unroll
-          for (int q = 0; q < NKQ; ++q) {
-            const uint4 v = sm.keys[((size_t)f * NKQ + q) * kThreads + tid];
-            const uint32_t kk[4] = {v.x, v.y, v.z, v.w};
-  #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              if (4 * q + i >= NK) continue;
-              bool sel = kk[i] > thr;
-              if (kk[i] == thr) {
-                const int g = f * SS + flat_in_face<S>(tid, 4 * q + i), w = g >> 5;
-                sel = (int)(sm.wpre[w] + __popc(sm.bits[w] & ((1u << (g & 31)) - 1u))) < remaining;
-              }
-              n_sel += sel;
-            }
-          }
-      uint32_t all_sel;
-      int slot = (int)block_inclusive_sum((uint32_t)n_sel, sm.warp_tot, &all_sel) - n_sel;
-      if (owner && n_sel)
-        for (int f = 0; f < 6; ++f)
-  #pragma unroll
-          for (int q = 0; q < NKQ; ++q) {
-            const uint4 v = sm.keys[((size_t)f * NKQ + q) * kThreads + tid];
-            const uint32_t kk[4] = {v.x, v.y, v.z, v.w};
-  #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              if (4 * q + i >= NK) continue;
-              const int u = 4 * q + i;
-              const int g = f * SS + flat_in_face<S>(tid, u);
-              bool sel = kk[i] > thr;
-              if (kk[i] == thr) {
-                const int w = g >> 5;
-                sel = (int)(sm.wpre[w] + __popc(sm.bits[w] & ((1u << (g & 31)) - 1u))) < remaining;
-              }
-              if (sel) {
-                sm.gkey[slot] = ((uint64_t)kk[i] << 32) | (uint64_t)(0xFFFFFFFFu - (uint32_t)g);
-                sm.gid[slot] = (f * NK + u) * kThreads + tid;
-                ++slot;
-              }
-            }
-          }
-      __syncthreads();
-    }
-    // ---- order the K winners.  Every winner's key lies in [prefix, kmax] (prefix: the window
-    // bin's lower edge or the exact threshold), so a counting pass over 256 bins of that range
-    // (bin 0 = the largest keys) places them, and each is ranked only among the few winners of
-    // its own bin by the composite key.  The histogram region is free again here.
-    uint32_t* bin_n = sm.whist;                                    // [256] winners per bin
-    uint32_t* bin_end = sm.whist + 256;                            // [256] scatter cursor
-    uint16_t* order = reinterpret_cast<uint16_t*>(sm.whist + 512);  // [K] winners by bin
-    const uint32_t range = kmax - prefix;
-    const int bshift = range < 256u ? 0 : 24 - __clz((int)range);  // (range >> bshift) < 256
-    auto bin_of = [&](uint64_t ck) { return (kmax - (uint32_t)(ck >> 32)) >> bshift; };
-    bin_n[tid] = 0u;  // kThreads == 256 bins
-    __syncthreads();
-    for (int e = tid; e < K; e += kThreads) atomicAdd(&bin_n[bin_of(sm.gkey[e])], 1u);
-    __syncthreads();
-    {
-      uint32_t all;
-      const uint32_t n = bin_n[tid];
-      bin_end[tid] = block_inclusive_sum(n, sm.warp_tot, &all) - n;  // starts; ends after the scatter
+      h4[0] = make_uint4(start[0], start[1], start[2], start[3]);
+      h4[1] = make_uint4(start[4], start[5], start[6], start[7]);
+      if (tid == 0) sm.hist[kBins] = 0u;  // the end of the part above the topmost bin's
+      if (tid == kThreads - 1 && all < (uint32_t)K) sm.scal[kScNAbove] = (int)all;
     }
     __syncthreads();
-    for (int e = tid; e < K; e += kThreads) order[atomicAdd(&bin_end[bin_of(sm.gkey[e])], 1u)] = (uint16_t)e;
-    __syncthreads();
-    for (int e = tid; e < K; e += kThreads) {
-      const uint64_t me = sm.gkey[e];
-      const uint32_t b = bin_of(me), end = bin_end[b];
-      int rank = (int)(end - bin_n[b]);
-      for (uint32_t i = end - bin_n[b]; i < end; ++i) rank += sm.gkey[order[i]] > me;
-      const int id = sm.gid[e];
+    const uint32_t lo_key = (uint32_t)sm.scal[kScPrefix];
+    int n_all = *n_listed, n_final = sm.scal[kScNAbove];
+    if (n_all > cap && n_final <= list_cap(K)) {
+      // the list overflowed (faces each brighter than the one before), but the counts are whole
+      list_again<S>(map, lo_key, K);
+      n_all = *n_listed;
+    }
+    const bool general = n_all > cap || n_final > list_cap(K);
+    if (!general) {
+      for (int e = tid; e < n_all; e += kThreads) {
+        const uint32_t k = sm.lkey[e];
+        if (k < lo_key) continue;
+        const int id = sm.lid[e], t = id % kThreads, fu = id / kThreads, f = fu / NK, u = fu % NK;
+        const int g = f * SS + flat_in_face<S>(t, u);
+        const uint32_t slot = atomicAdd(&sm.hist[k >> 20], 1u);
+        sm.gkey[slot] = ((uint64_t)k << 32) | (uint64_t)(0xFFFFFFFFu - (uint32_t)g);
+        sm.gid[slot] = (uint16_t)id;
+      }
+      __syncthreads();
+    } else {
+      general_select<S>(map, K);
+      n_final = K;
+    }
+    // one channel of a winner: its strength (and, with the first, its index)
+    auto put = [&](int rank, int c, int id) {
       const int t = id % kThreads, fu = id / kThreads, f = fu / NK, u = fu % NK;
       const size_t out = (size_t)env * K + rank;
-      float v[3] = {0.f, 0.f, 0.f};
-      if (u == NR) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) v[c] = up[(f * 3 + c) * kThreads + t];
-      } else if constexpr (NR > 0) {
-        block_coef<S>(faces + ((size_t)env * 6 + f) * (size_t)SS * 3, t, u, v);
-      }
-      idx_out[out] = f * SS + flat_in_face<S>(t, u);
-      st_out[out * 3 + 0] = v[0];
-      st_out[out * 3 + 1] = v[1];
-      st_out[out * 3 + 2] = v[2];
+      float v = 0.f;
+      if (u == NR) v = up[(f * 3 + c) * kThreads + t];
+      else if constexpr (NR > 0) v = block_coef<S>(map + (size_t)f * SS * 3, t, u, c);
+      if (c == 0) idx_out[out] = f * SS + flat_in_face<S>(t, u);
+      st_out[out * 3 + c] = v;
+    };
+    for (int e = tid; e < n_final; e += kThreads) {
+      const uint64_t me = sm.gkey[e];
+      // its bin's part ends where the bin's next key would go, and starts where the bin above ends
+      const uint32_t bin = (uint32_t)(me >> 52);
+      int rank = general ? 0 : (int)sm.hist[bin + 1];
+      const uint64_t* o = sm.gkey + rank;
+      const int n = (general ? K : (int)sm.hist[bin]) - rank;
+#pragma unroll 4
+      for (int i = 0; i < n; ++i) rank += o[i] > me;
+      if (rank < K) sm.order[rank] = sm.gid[e];
     }
-    __syncthreads();  // the next map reuses every shared array and the scratch slice
+    if (n_final < K) {
+      // ---- fewer than K keys above 0: then the coefficients not listed, in flat-index order
+      constexpr int NW = (6 * SS + 31) / 32, PER = (NW + kThreads - 1) / kThreads;
+      for (int w = tid; w < NW; w += kThreads) sm.bits[w] = w * 32 + 32 <= 6 * SS ? 0u : ~0u << (6 * SS - w * 32);
+      __syncthreads();
+      for (int e = tid; e < n_final; e += kThreads) {
+        const uint32_t g = 0xFFFFFFFFu - (uint32_t)sm.gkey[e];
+        atomicOr(&sm.bits[g >> 5], 1u << (g & 31));
+      }
+      __syncthreads();
+      uint32_t mine = 0, all;
+      for (int i = 0; i < PER; ++i) mine += tid * PER + i < NW ? 32u - (uint32_t)__popc(sm.bits[tid * PER + i]) : 0u;
+      uint32_t run = block_inclusive_sum(mine, sm.warp_tot, &all) - mine;
+      for (int i = 0; i < PER; ++i)
+        if (tid * PER + i < NW) {
+          sm.wpre[tid * PER + i] = run;
+          run += 32u - (uint32_t)__popc(sm.bits[tid * PER + i]);
+        }
+      __syncthreads();
+      for (int w = warp; w < NW && n_final + (int)sm.wpre[w] < K; w += kWarps) {
+        const uint32_t z = ~sm.bits[w];
+        const int rank = n_final + (int)sm.wpre[w] + __popc(z & ((1u << lane) - 1u));
+        if ((z >> lane & 1u) && rank < K) sm.order[rank] = (uint16_t)id_of_flat<S>(w * 32 + lane);
+      }
+    }
+    __syncthreads();
+    for (int i = tid; i < 3 * K; i += kThreads) put(i / 3, i % 3, sm.order[i / 3]);
+    __syncthreads();  // the next map reuses every shared array
   }
 }
 
 // Batches of at least this many maps use the batched kernel; smaller ones the cluster form.  48
-// clusters of six run at once on 148 SMs, so 96 maps are two rounds of it; the batched kernel takes
-// the same time for 1 to 148 maps.  us at S = 64, K = 300 (K = 1024), cluster form and batched:
-// 32 maps 8.9 and 23.9 (13.3, 33.4), 64 maps 16.5 and 24.0 (24.6, 33.5), 98 maps 23.8 and 24.1
-// (35.0, 33.6), 147 maps 32.3 and 25.9 (48.0, 34.2).
-constexpr int kBatchMinMaps = 97;
-
-// A stream-ordered pool per device for the batched kernel's scratch.  It keeps its memory
-// between calls (release threshold = max), so a steady stream of batches allocates once.
-std::mutex g_pool_mu;
-cudaMemPool_t g_pool[64] = {};
-
-cudaMemPool_t scratch_pool(int dev) {
-  std::lock_guard<std::mutex> lock(g_pool_mu);
-  if (dev < 0 || dev >= 64) fail(NWPRT_UNSUPPORTED, "haar_topk: device ordinal beyond the pool table");
-  if (!g_pool[dev]) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t pool;
-    NWPRT_CUDA(cudaMemPoolCreate(&pool, &props));
-    uint64_t keep = ~0ull;
-    NWPRT_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-    g_pool[dev] = pool;
-  }
-  return g_pool[dev];
-}
+// clusters of six run at once on 148 SMs, so the cluster form's time grows every 48 maps; the
+// batched kernel takes the same time for 1 to 148 maps (one per SM), which grows with K and, its
+// block holding several small faces at once, falls with S.  us, cluster form and batched:
+//   S = 64, K = 300    48 maps  9.0 and 24.9    96 maps 17.5 and 24.9    98 maps 23.8 and 24.9
+//   S = 64, K = 1024   96 maps  26  and 41.5   128 maps 37.3 and 41.5   144 maps 47.7 and 41.8
+//   S = 32, K = 300    64 maps 13.1 and 14.4    97 maps 18.6 and 14.4
+//   S = 16, K = 64     32 maps  5.6 and  7.2    49 maps  9.5 and  7.2
+int batch_min_maps(int S, int K) { return S <= 16 ? 49 : (K > 512 ? 129 : 97); }
 
 template <int S>
 void launch_s(const float* faces, int n_env, int K, int32_t* idx, float* strength, cudaStream_t st) {
@@ -1180,22 +1281,15 @@ void launch_s(const float* faces, int n_env, int K, int32_t* idx, float* strengt
   NWPRT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   NWPRT_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const size_t bsmem = batch_smem_layout(S, K, nullptr, nullptr);
-  if (n_env >= kBatchMinMaps && bsmem <= (size_t)max_smem) {
+  if (n_env >= batch_min_maps(S, K) && bsmem <= (size_t)max_smem) {
     NWPRT_CUDA(cudaFuncSetAttribute(haar_topk_batch_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
     int per_sm = 0;
     NWPRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, haar_topk_batch_kernel<S>, kThreads, bsmem));
     const long long slots = (long long)sms * (per_sm > 0 ? per_sm : 1);
     const int grid = (int)(n_env < slots ? n_env : slots);
-    void* scratch = nullptr;
-    const size_t bytes = (size_t)grid * batch_scratch_floats_per_cta<S>() * sizeof(float);
-    if (cudaMallocFromPoolAsync(&scratch, bytes, scratch_pool(dev), st) == cudaSuccess) {
-      haar_topk_batch_kernel<S><<<grid, kThreads, bsmem, st>>>(faces, n_env, K, idx, strength, (float*)scratch);
-      const cudaError_t launch = cudaGetLastError();
-      NWPRT_CUDA(cudaFreeAsync(scratch, st));
-      NWPRT_CUDA(launch);
-      return;
-    }
-    (void)cudaGetLastError();  // no scratch: the cluster form needs none
+    haar_topk_batch_kernel<S><<<grid, kThreads, bsmem, st>>>(faces, n_env, K, idx, strength);
+    NWPRT_CUDA(cudaGetLastError());
+    return;
   }
   const size_t smem = smem_layout(S, K, nullptr, nullptr);
   NWPRT_CUDA(cudaFuncSetAttribute(haar_topk_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -1,6 +1,6 @@
-"""GPU tests of the two Haar + top-K forms on either side of the batch size that separates them
-(a cluster per map up to 96 maps, a persistent CTA per map from 97), bit for bit against the
-oracle, on maps that take each form's shortcuts and their fallbacks."""
+"""GPU tests of the two Haar + top-K forms on either side of the batch sizes that separate them (a
+cluster per map, or a persistent CTA per map from 49, 97 or 129 maps, by face size and K), bit for
+bit against the oracle, on maps that take each form's shortcuts and their fallbacks."""
 import numpy as np
 import pytest
 
@@ -29,6 +29,9 @@ def _maps(S, K, E):
         lambda m: m.__imul__(1e-38),                                             # subnormal keys
         lambda m: m.__imul__(np.float32(2.0) ** np.arange(-30, 30)[g.integers(0, 60, m.shape)]),  # wide range
         lambda m: m.__setitem__(slice(1, 6), 0.0),                               # one face holds everything
+        lambda m: m.__imul__(np.float32(10.0) ** np.arange(6, dtype=np.float32).reshape(6, 1, 1, 1)),  # ever brighter
+        lambda m: m.__imul__(np.float32(0.1) ** np.arange(6, dtype=np.float32).reshape(6, 1, 1, 1)),   # ever darker
+        lambda m: m.__imul__(g.random(m.shape[:3] + (1,)) < 3e-3),               # few lights on black
     ]
     for i, edit in enumerate(edits):
         if 2 * i + 1 < E:
@@ -38,7 +41,7 @@ def _maps(S, K, E):
 
 @pytest.mark.parametrize("S,K", [(64, 300), (64, 1), (64, 1024), (32, 64), (32, 1024), (16, 300), (8, 384), (4, 96),
                                  (2, 24), (1, 6)])
-@pytest.mark.parametrize("E", [1, 25, 96, 97, 310])
+@pytest.mark.parametrize("E", [1, 25, 48, 49, 96, 97, 128, 129, 310])
 def test_haar_topk_forms_bit_exact(cuda, S, K, E):
     import torch
     from neural_wavelet_prt_demo_b200 import engine as eng
