@@ -128,9 +128,7 @@ __device__ __forceinline__ uint32_t wavelet_key_bits(float r, float g, float b) 
   float t = __fmul_rn(0.212671f, r);
   t = __fadd_rn(t, __fmul_rn(0.715160f, g));
   t = __fadd_rn(t, __fmul_rn(0.072169f, b));
-  t = fabsf(t);
-  if (t != t) t = 0.0f;
-  return __float_as_uint(t);
+  return __float_as_uint(fmaxf(fabsf(t), 0.0f));  // the maximum of NaN and 0 is 0
 }
 
 // Bits 0, 2, 4, 6 of x packed into bits 0..3 (Morton decode of one coordinate).
@@ -696,11 +694,11 @@ __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
 // (general_select).
 //
 // Small faces share the block: FPI of them are transformed at once.  Bound by latency and issue:
-// four CTAs of 64 registers fit an SM (1.09 us per map and SM slot), and what they leave of the
+// four CTAs of 64 registers fit an SM (109 us for 1,024 maps), and what they leave of the
 // SM's memory as L1 matters, since a texel row's three 16-byte loads share their sectors (lists of
 // 6 K + 768 keys instead of 5 K + 512 took one step of it: 110 -> 117 us).  1,024 maps, K = 300:
-// 132 us -> 110 (2,790 GB/s) with all keys kept in shared memory, three scans of them and two CTAs
-// per SM before; K = 64 109 -> 88, K = 1024 229 -> 208; S = 32 102 -> 50; S = 16, K = 64 67 -> 19;
+// 132 us -> 109 (2,820 GB/s) with all keys kept in shared memory, three scans of them and two CTAs
+// per SM before; K = 64 109 -> 87, K = 1024 229 -> 206; S = 32 102 -> 50; S = 16, K = 64 67 -> 19;
 // maps of few lights on black 269 -> 84.  Each face ten times brighter than the one before is the
 // bad case: 121 -> 174.
 
