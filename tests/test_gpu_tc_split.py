@@ -48,3 +48,40 @@ def test_shared_and_whole_tiles_give_the_same_bits(cuda, cfg, K, kahan):
     for got, ref in zip((fr.fbPredictedIndirect, fr.fbPredictedIndirectWithDirect), whole):
         assert np.array_equal(got.cpu().numpy().view(np.uint32), ref.view(np.uint32))
     e.close()
+
+
+@pytest.mark.parametrize("net,precision,K", [("six", "fp8", 13), ("two", "fp8", 40), ("plan", "fp8", 13),
+                                             ("plan", "bf16", 11)])
+def test_split_without_the_tensor_core_output_layer(cuda, net, precision, K):
+    # the forms that sum T_k in the last layer's epilogue: a frame of 740 whole tiles and 34 shared
+    # ones against its first rows alone, whose tiles are all shared (1 per SM, then 2)
+    import copy
+    import dataclasses
+
+    from neural_wavelet_prt_demo_b200 import engine as eng
+    cfg = copy.deepcopy(netconfig.CONFIG_SMALL if net == "two" else netconfig.CONFIG_LARGE)
+    if net == "plan":  # five layers: read from the plan at run time
+        cfg["out_prd"]["n_hidden_layers"] = cfg["cmp_net"]["n_hidden_layers"] = 2
+    case = make_case(cfg, 1021, 97, K, seed=K, hash_scale=0.5, flag_prob=0.9)
+    e = eng.RenderEngine(case.cfg)
+    e.loadWeights(case.weights)
+    env = e.addEnvironmentMap(eng.EnvironmentMap(top_coefficients=case.idx, top_strength=case.strength))
+    rc = eng.RenderConfig(precision=precision)
+    out = []
+    for rows in (97, 18, 30):
+        n = 1021 * rows
+        gb = dataclasses.replace(case.gbuf, height=rows, **{
+            f: getattr(case.gbuf, f)[:n] for f in ("pos", "normal", "reflect", "roughness", "kd", "ks", "direct", "flag")})
+        fr = eng.FullFrame.from_gbuffer(gb)
+        e.setFrame(0, fr)
+        e.TCNNPass_p1(0)
+        if precision == "fp8" and not out:
+            e.calibrateFP8(env, 0)
+        e.TCNNPass_p2(env, 0, rc)
+        e.TCNNSync()
+        out.append(fr.fbPredictedIndirect.cpu().numpy())
+    assert psnr(out[0][:, :3], O.relight_f64(case.bound, case.idx, case.strength)) >= (30.0 if precision == "fp8"
+                                                                                       else PSNR_MIN)
+    for part in out[1:]:
+        assert np.array_equal(part.view(np.uint32), out[0][:len(part)].view(np.uint32))
+    e.close()
