@@ -436,6 +436,7 @@ __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
   HaarSmem sm;
   smem_layout(S, K, smem_raw, &sm);
   cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();  // waited for before the first store to another CTA, which must have started
   const int face = (int)cluster.block_rank();
   const int env = blockIdx.x / 6;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -472,6 +473,7 @@ __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
 #pragma unroll
       for (int u = 0; u < NK; ++u) m = max(m, key[u]);
     m = __reduce_max_sync(0xffffffffu, m);
+    cluster.barrier_wait();
     if (lane < 6) cluster.map_shared_rank(sm.kmax, lane)[face * kWarps + warp] = m;
   }
   cluster.sync();
