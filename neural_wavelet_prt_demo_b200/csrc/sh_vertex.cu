@@ -78,6 +78,8 @@ __global__ void __launch_bounds__(kWarps * 32) sh_vertex_kernel(const float* __r
       const int head = ((4 - mis) & 3) < nn ? ((4 - mis) & 3) : nn;
       const int body = (nn - head) & ~3;
       if (lane == 0) {
+        // a head or tail of the matrix before, written by cp.async, may lie where this copy writes
+        fence_proxy_async_smem();
         mbar_arrive_expect_tx(&full[warp], body * 4);
         if (body > 0) bulk_g2s(t + head, src + head, body * 4, &full[warp]);
       }
