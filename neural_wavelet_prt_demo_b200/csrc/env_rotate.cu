@@ -30,6 +30,7 @@ __device__ __forceinline__ void uv_to_dir(int f, float uc, float vc, float& x, f
 }
 
 __global__ void env_rotate_kernel(const float* __restrict__ src, int S, Rot R, float* __restrict__ dst) {
+  let_next_start();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long SS = (long long)S * S;
   if (t >= 6 * SS) return;
@@ -64,6 +65,7 @@ __global__ void env_rotate_kernel(const float* __restrict__ src, int S, Rot R, f
   row %= S;
   if (col < 0) col += S;
   if (row < 0) row += S;
+  stream_wait(src, dst);
   const float* s = src + (((long long)sf * S + row) * S + col) * 3;
   float* d = dst + t * 3;
   d[0] = s[0];
@@ -84,7 +86,7 @@ void launch_env_rotate(const float* src, int S, const float* R_host, float* dst,
     R.m[i] = R_host[i];
   }
   const long long n = 6LL * S * S;
-  env_rotate_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(src, S, R, dst);
+  launch_overlapped(env_rotate_kernel, (n + 255) / 256, 256, 0, st, src, S, R, dst);
   NWPRT_CUDA(cudaGetLastError());
 }
 

@@ -440,7 +440,6 @@ __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
   const int face = (int)cluster.block_rank();
   const int env = blockIdx.x / 6;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const float* src = faces + ((size_t)env * 6 + face) * (size_t)SS * 3;
   const bool owner = tid < T;
 
   if (face == 0 && tid == 0) sm.scal[kScCounter] = 0;  // winner slots (read after 5 cluster barriers)
@@ -448,6 +447,9 @@ __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
   sm.hist[tid] = 0u;                     // kThreads == 256 bins
   if (tid == 0) sm.scal[kScListed] = -1;  // stays when the window holds fewer than K keys
   // (barriers in the transform order these)
+  let_next_start();
+  stream_wait(faces, idx_out, st_out);
+  const float* src = faces + ((size_t)env * 6 + face) * (size_t)SS * 3;
 
   // ---- the transform: levels 1-2 in registers, the rest by shuffles and warp 0
   float co[NR > 0 ? NR : 1][3];  // detail coefficients held in registers (RGB)
@@ -1069,6 +1071,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
   const int cap = face_list_cap(S, K);
   float* up = sm.up;
   int* n_listed = &sm.scal[kScListed];
+  stream_wait(faces, idx_out, st_out);
 
   for (int env = blockIdx.x; env < n_env; env += gridDim.x) {
     const float* map = faces + (size_t)env * 6 * SS * 3;
@@ -1287,13 +1290,13 @@ void launch_s(const float* faces, int n_env, int K, int32_t* idx, float* strengt
     NWPRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, haar_topk_batch_kernel<S>, kThreads, bsmem));
     const long long slots = (long long)sms * (per_sm > 0 ? per_sm : 1);
     const int grid = (int)(n_env < slots ? n_env : slots);
-    haar_topk_batch_kernel<S><<<grid, kThreads, bsmem, st>>>(faces, n_env, K, idx, strength);
+    launch_overlapped(haar_topk_batch_kernel<S>, grid, kThreads, bsmem, st, faces, n_env, K, idx, strength);
     NWPRT_CUDA(cudaGetLastError());
     return;
   }
   const size_t smem = smem_layout(S, K, nullptr, nullptr);
   NWPRT_CUDA(cudaFuncSetAttribute(haar_topk_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  haar_topk_kernel<S><<<6 * n_env, kThreads, smem, st>>>(faces, K, idx, strength);
+  launch_overlapped(haar_topk_kernel<S>, 6LL * n_env, kThreads, smem, st, faces, K, idx, strength);
   NWPRT_CUDA(cudaGetLastError());
 }
 

@@ -21,6 +21,8 @@ __global__ void pack_gbuffer_kernel(int64_t n, const float4* __restrict__ pos,
                                     const float* __restrict__ rough, const float4* __restrict__ kd,
                                     const float4* __restrict__ ks, float rgh_den,
                                     float4* __restrict__ out) {
+  let_next_start();
+  stream_wait(pos, nrm, refl, rough, kd, ks, out);
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
   const float4 a = pos[p], b = nrm[p], c = refl[p], d = kd[p], e = ks[p];
@@ -35,6 +37,8 @@ __global__ void pack_gbuffer_kernel(int64_t n, const float4* __restrict__ pos,
 __global__ void gather_embedding_kernel(const float* __restrict__ emb, int D, int n_coeffs,
                                         const int32_t* __restrict__ idx, int K,
                                         float* __restrict__ out, uint32_t* __restrict__ out_h, uint32_t* err) {
+  let_next_start();
+  stream_wait(emb, idx, out, out_h);
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int H = D / 2;
   if (t >= (int64_t)K * H) return;
@@ -64,8 +68,8 @@ void launch_pack_gbuffer(const nwprt_gbuffer& g, float* packed, cudaStream_t st)
   // the reference's constant 1/log(26) (utils_kernels.h:21), evaluated once on the host
   const float rgh_den = 1.f / logf_series(25.f + 1.f);
   const int bs = 256;
-  pack_gbuffer_kernel<<<(unsigned)((n + bs - 1) / bs), bs, 0, st>>>(
-      n, (const float4*)g.first_hit_pos, (const float4*)g.world_normal, (const float4*)g.reflect_dir,
+  launch_overlapped(
+      pack_gbuffer_kernel, (n + bs - 1) / bs, bs, 0, st, n, (const float4*)g.first_hit_pos, (const float4*)g.world_normal, (const float4*)g.reflect_dir,
       g.roughness, (const float4*)g.kd, (const float4*)g.ks, rgh_den, (float4*)packed);
   NWPRT_CUDA(cudaGetLastError());
 }
@@ -75,8 +79,7 @@ void launch_gather_embedding(const float* emb, int D, int n_coeffs, const int32_
   if (D % 2) fail(NWPRT_UNSUPPORTED, "embedding gather needs an even feature count");
   const int64_t n = (int64_t)K * (D / 2);
   if (n == 0) return;
-  gather_embedding_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(emb, D, n_coeffs, idx, K,
-                                                                        out_kd, out_h, err);
+  launch_overlapped(gather_embedding_kernel, (n + 255) / 256, 256, 0, st, emb, D, n_coeffs, idx, K, out_kd, out_h, err);
   NWPRT_CUDA(cudaGetLastError());
 }
 

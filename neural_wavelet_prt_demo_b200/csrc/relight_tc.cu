@@ -741,6 +741,7 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  stream_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1520,7 +1521,7 @@ void launch_relight_tc(const NetDims& d, const HashLevels& hl, const float* hash
   auto go = [&](auto kern) {
     NWPRT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (counted) NWPRT_CUDA(cudaMemsetAsync(tile_ctr, 0, sizeof(int), st));
-    kern<<<grid, kThreads, smem, st>>>(p);
+    launch_overlapped(kern, grid, kThreads, smem, st, p);
   };
   const int shape = shape_of(P, d);
   if (mode == kTcBf16 && shape != kShapePlan && (P.out_k != 64 || P.out_sbo == 0))

@@ -113,6 +113,8 @@ __global__ void __launch_bounds__(kProjThreads) sh_project_partial(const float* 
   const long long SS = (long long)S * S;
   const int grp = tid % kProjGroup, slice = tid / kProjGroup;
   float acc[3][3] = {};
+  let_next_start();
+  stream_wait(faces, part);
   for (int chunk = blockIdx.x; chunk < n_chunks; chunk += gridDim.x) {
     const long long t = (long long)chunk * kProjThreads + tid;
     if (t < 6 * SS) {
@@ -183,6 +185,7 @@ __global__ void __launch_bounds__(1024) sh_project_reduce(const float* __restric
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int o = blockIdx.x * 32 + lane;
   float acc = 0.f;
+  stream_wait(part, L);
   if (o < kNc * 3)
 #pragma unroll 8
     for (int b = warp; b < n_blocks; b += 32) acc += part[(size_t)b * (kNc * 3) + o];
@@ -288,9 +291,9 @@ void launch_sh_project(const float* faces, int S, float* L, float* workspace, cu
   NWPRT_CUDA(cudaGetDevice(&dev));
   NWPRT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int grid = chunks < 2 * sms ? chunks : 2 * sms;  // two blocks fit an SM
-  sh_project_partial<<<grid, kProjThreads, kProjSmem, st>>>(faces, S, chunks, workspace);
+  launch_overlapped(sh_project_partial, grid, kProjThreads, kProjSmem, st, faces, S, chunks, workspace);
   NWPRT_CUDA(cudaGetLastError());
-  sh_project_reduce<<<(kNc * 3 + 31) / 32, 1024, 0, st>>>(workspace, grid, L);
+  launch_overlapped(sh_project_reduce, (kNc * 3 + 31) / 32, 1024, 0, st, workspace, grid, L);
   NWPRT_CUDA(cudaGetLastError());
 }
 

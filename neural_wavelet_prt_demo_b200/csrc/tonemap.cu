@@ -66,6 +66,8 @@ __global__ void __launch_bounds__(256) tonemap_srgb_kernel(const __grid_constant
   asm volatile("" : "+l"(table));  // one coalesced load, not 32 constant-bank reads per warp
   t[threadIdx.x] = table[threadIdx.x];
   __syncthreads();
+  let_next_start();
+  stream_wait(src, dst);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const float4 v = __ldg(src + i);
     dst[i] = lookup(t, v.x) | (lookup(t, v.y) << 8) | (lookup(t, v.z) << 16) | (255u << 24);
@@ -84,8 +86,8 @@ void launch_tonemap_srgb(const float* src, int64_t n, uint32_t* dst, cudaStream_
   NWPRT_CUDA(cudaGetDevice(&dev));
   NWPRT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int64_t blocks = (n + 255) / 256, cap = (int64_t)sms * 8;
-  tonemap_srgb_kernel<<<(int)(blocks < cap ? blocks : cap), 256, 0, st>>>(
-      table(), reinterpret_cast<const float4*>(src), n, dst);
+  launch_overlapped(tonemap_srgb_kernel, blocks < cap ? blocks : cap, 256, 0, st, table(),
+                    reinterpret_cast<const float4*>(src), n, dst);
   NWPRT_CUDA(cudaGetLastError());
 }
 
