@@ -77,6 +77,7 @@ struct HaarSmem {
 constexpr int kScPrefix = 0, kScMask = 1, kScRemaining = 2, kScCounter = 3, kScEq = 8;  // eq: [6]
 constexpr int kScListed = 14;                // cluster form: keys listed
 constexpr int kScNAbove = 16;                // batched kernel: keys in the final list
+constexpr int kScLevels = 17;                // batched kernel: winners written so far, those of level 2 apart: [2]
 
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
@@ -697,14 +698,15 @@ __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
 // too full (hundreds of equal keys) recomputes its keys in each pass of a radix select
 // (general_select).
 //
-// Small faces share the block: FPI of them are transformed at once.  Bound by latency and issue:
-// four CTAs of 64 registers fit an SM (109 us for 1,024 maps), and what they leave of the
+// Small faces share the block: FPI of them are transformed at once.  Bound by L1 (69% busy) and issue
+// (63%): four CTAs of 64 registers fit an SM (107 us for 1,024 maps), and what they leave of the
 // SM's memory as L1 matters, since a texel row's three 16-byte loads share their sectors (lists of
 // 6 K + 768 keys instead of 5 K + 512 took one step of it: 110 -> 117 us).  1,024 maps, K = 300:
-// 132 us -> 109 (2,820 GB/s) with all keys kept in shared memory, three scans of them and two CTAs
-// per SM before; K = 64 109 -> 87, K = 1024 229 -> 206; S = 32 102 -> 50; S = 16, K = 64 67 -> 19;
+// 132 us -> 107 (2,870 GB/s) with all keys kept in shared memory, three scans of them and two CTAs
+// per SM before; K = 64 109 -> 86, K = 1024 229 -> 202; S = 32 102 -> 50; S = 16, K = 64 67 -> 19;
 // maps of few lights on black 269 -> 84.  Each face ten times brighter than the one before is the
-// bad case: 121 -> 174.
+// bad case: 121 -> 174.  Of these, one prefix sum per list instead of a ballot per key and writing the
+// level-2 winners apart give 109.4 -> 107.1 (K = 64 86.4 -> 85.9, K = 1024 208.8 -> 202.3).
 
 constexpr int kBins = 2048;       // of keys by bits 30..20
 constexpr int kCtasPerSm = 4;
@@ -724,6 +726,7 @@ struct BatchSmem {
   uint64_t* gkey;   // [list_cap] composite keys of the final list
   uint16_t* gid;    // [list_cap]
   uint16_t* order;  // [K] aliases lid: the winners' coefficients by rank
+  uint16_t* turn;   // [K] aliases lkey: their ranks in the order they are written
   float* up;        // [6][3][kThreads] the upper-block entries: [face][channel][thread]
   float* llg;       // [6][16][3] each face's LL values left for its last levels
   int* warp_tot;
@@ -748,6 +751,7 @@ __host__ __device__ inline size_t batch_smem_layout(int S, int K, char* base, Ba
     L->hist = (uint32_t*)(base + oH);
     L->up = (float*)(base + oU);
     L->order = (uint16_t*)(base + oI);
+    L->turn = (uint16_t*)(base + oL);
     L->lkey = (uint32_t*)(base + oL);
     L->bits = (uint32_t*)(base + oL);
     L->wpre = (uint32_t*)(base + oL) + nw;
@@ -924,22 +928,29 @@ struct KeyList {
       counted = true;
     }
     if (total == 0) return;
-    int at = 0;
-    if (lane == 0) at = atomicAdd(&sm.scal[kScListed], total);
-    at = __shfl_sync(0xffffffffu, at, 0);
-    crowded |= at > 4 * K + 384;
+    // each lane's hits go side by side, after those of the lanes below it
+    int at = __popc(hits);
 #pragma unroll
-    for (int u = 0; u < N; ++u) {
-      const bool h = hits >> u & 1u;
-      const uint32_t b = __ballot_sync(0xffffffffu, h);
-      const int p = at + __popc(b & ((1u << lane) - 1u));
-      if (h && p < cap) {
-        sm.lkey[p] = k[u];
-        sm.lid[p] = (uint16_t)id(u);
-      }
-      if (h && !counted) atomicAdd(&sm.hist[k[u] >> 20], 1u);  // also past the list's end
-      at += __popc(b);
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, at, o);
+      if (lane >= o) at += t;
     }
+    int base = 0;
+    if (lane == 31) base = atomicAdd(&sm.scal[kScListed], total);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    crowded |= base > 4 * K + 384;
+    at += base - __popc(hits);
+    const bool count = !counted, room = base + total <= cap;
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+      if (hits >> u & 1u) {
+        if (room || at < cap) {
+          sm.lkey[at] = k[u];
+          sm.lid[at] = (uint16_t)id(u);
+        }
+        if (count) atomicAdd(&sm.hist[k[u] >> 20], 1u);  // also past the list's end
+        ++at;
+      }
   }
 };
 
@@ -1163,6 +1174,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     if (tid == 0) {
       sm.scal[kScPrefix] = 1;  // every listed key, if they are fewer than K
       sm.scal[kScNAbove] = -1;
+      sm.scal[kScLevels] = sm.scal[kScLevels + 1] = 0;
     }
     __syncthreads();
     // ---- the last winner's bin: eight bins a thread from the top.  A bin's part of the final list
@@ -1262,7 +1274,23 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       }
     }
     __syncthreads();
-    for (int i = tid; i < 3 * K; i += kThreads) put(i / 3, i % 3, sm.order[i / 3]);
+    if constexpr (F::B == 4) {
+      // ---- the level-2 winners, which take four quads' texels, last: few warps then run both levels' code
+      for (int i0 = warp * 32; i0 < K; i0 += kThreads) {
+        const int i = i0 + lane, u = i < K ? sm.order[i] / kThreads % NK : 0;
+        const bool second = u >= 12 && u < NR;
+        const uint32_t in = __ballot_sync(0xffffffffu, i < K), b2 = __ballot_sync(0xffffffffu, second), b1 = in & ~b2;
+        int at = 0;
+        if (lane < 2) at = atomicAdd(&sm.scal[kScLevels + lane], __popc(lane ? b2 : b1));
+        const int a1 = __shfl_sync(0xffffffffu, at, 0), a2 = __shfl_sync(0xffffffffu, at, 1);
+        const uint32_t below = (1u << lane) - 1u;
+        if (i < K) sm.turn[second ? K - 1 - a2 - __popc(b2 & below) : a1 + __popc(b1 & below)] = (uint16_t)i;
+      }
+      __syncthreads();
+      for (int i = tid; i < 3 * K; i += kThreads) put(sm.turn[i / 3], i % 3, sm.order[sm.turn[i / 3]]);
+    } else {
+      for (int i = tid; i < 3 * K; i += kThreads) put(i / 3, i % 3, sm.order[i / 3]);
+    }
     __syncthreads();  // the next map reuses every shared array
   }
 }
