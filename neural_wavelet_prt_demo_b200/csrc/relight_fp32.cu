@@ -28,7 +28,7 @@ namespace nwprt {
 namespace {
 
 constexpr int r4(int x) { return (x + 3) & ~3; }
-constexpr int kMaxKChunk = 16;
+constexpr int kMaxKChunk = 16;  // most wavelets whose embedding rows and strengths a block holds at a time
 
 struct Fp32Params {
   HashLevels hl;
@@ -41,6 +41,7 @@ struct Fp32Params {
   const float* emb_k;
   const float* strength;
   int K;
+  int k_chunk;             // blocks of 32 pixels: the wavelets held at a time (others hold kMaxKChunk)
   int64_t px_begin, n_px;  // pixel range [px_begin, n_px)
   float* indirect;
   float* with_direct;
@@ -245,8 +246,9 @@ __global__ void __launch_bounds__(NT / WP * 32, 1) relight_fp32_kernel(const __g
   extern __shared__ __align__(16) float sm[];
   float* sW = sm;
   float* sE = sW + p.w_floats;
-  float* sL = sE + kMaxKChunk * g.d;
-  float* sAct = sL + kMaxKChunk * 4;
+  const int k_chunk = NT == 32 ? p.k_chunk : kMaxKChunk;  // a constant where it can be: 0.5% of the pass
+  float* sL = sE + r4(k_chunk * g.d);
+  float* sAct = sL + k_chunk * 4;
   const int tid = threadIdx.x, lane = tid & 31;
   for (int i = tid * 4; i < p.w_floats; i += kThreads * 4)
     *reinterpret_cast<float4*>(sW + i) = __ldg(reinterpret_cast<const float4*>(p.w + i));
@@ -272,8 +274,8 @@ __global__ void __launch_bounds__(NT / WP * 32, 1) relight_fp32_kernel(const __g
     }
   }
   float s[3] = {0.f, 0.f, 0.f}, comp[3] = {0.f, 0.f, 0.f};
-  for (int k0 = 0; k0 < p.K; k0 += kMaxKChunk) {
-    const int kc = min(kMaxKChunk, p.K - k0);
+  for (int k0 = 0; k0 < p.K; k0 += k_chunk) {
+    const int kc = min(k_chunk, p.K - k0);
     __syncthreads();
     for (int i = tid; i < kc * g.d; i += kThreads) sE[i] = p.emb_k[(size_t)k0 * g.d + i];
     for (int i = tid; i < kc * 3; i += kThreads) sL[(i / 3) * 4 + i % 3] = p.strength[(size_t)k0 * 3 + i];
@@ -364,14 +366,14 @@ bool net_seq(const NetDims& d, int max_smem, NetSeq* g, std::string* why) {
   return true;
 }
 
-size_t net_smem_bytes(const NetSeq& g, int w_floats, int nt) {
-  return sizeof(float) * ((size_t)w_floats + kMaxKChunk * g.d + kMaxKChunk * 4 + (size_t)g.rows * nt);
+size_t net_smem_bytes(const NetSeq& g, int w_floats, int nt, int k_chunk) {
+  return sizeof(float) * ((size_t)w_floats + r4(k_chunk * g.d) + k_chunk * 4 + (size_t)g.rows * nt);
 }
 
 template <int NT, int WP>
 void launch_nt(const Fp32Params& p, const NetSeq& g, cudaStream_t st) {
   auto k = relight_fp32_kernel<NT, WP>;
-  const size_t smem = net_smem_bytes(g, p.w_floats, NT);
+  const size_t smem = net_smem_bytes(g, p.w_floats, NT, p.k_chunk);
   NWPRT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int64_t n = p.n_px - p.px_begin;
   k<<<(unsigned)((n + NT - 1) / NT), NT / WP * 32, smem, st>>>(p, g);
@@ -429,7 +431,8 @@ void launch_relight_fp32(const NetDims& d, const HashLevels& hl, const DeviceWei
   const NetLayer& last = g.l[g.n - 1];
   if (last.w_off + last.in * w_stride(last.out, true) != p.w_floats) fail(NWPRT_INVALID_ARG, "fp32 weight layout mismatch");
   const int64_t n = p.n_px - p.px_begin;
-  auto fits = [&](int nt) { return net_smem_bytes(g, p.w_floats, nt) <= (size_t)max_smem; };
+  p.k_chunk = kMaxKChunk;
+  auto fits = [&](int nt) { return net_smem_bytes(g, p.w_floats, nt, p.k_chunk) <= (size_t)max_smem; };
   // Pixels per block (mostly one block per SM at a time, as its weights and activations fill the
   // shared memory).  Blocks of 256 and more give a warp 32 pixels, smaller ones 16: half the
   // arithmetic per weight read, twice the warps.  us of one round of 148 blocks at K = 64:
@@ -446,7 +449,13 @@ void launch_relight_fp32(const NetDims& d, const HashLevels& hl, const DeviceWei
     const double c = (double)(((n + f.nt - 1) / f.nt + sms - 1) / sms) * f.cost;
     if (!nt || c < best) nt = f.nt, best = c;
   }
-  if (!nt && fits(32)) nt = 32;
+  if (!nt) {
+    // A block of 32 pixels, with as many wavelets at a time as fit.  Padded weight rows can take more
+    // than the smaller block saves (two deep networks 33 to 46 wide behind some 160 hash features and
+    // more), but one wavelet at a time fits every network that net_seq accepts.
+    while (p.k_chunk > 1 && !fits(32)) p.k_chunk /= 2;
+    if (fits(32)) nt = 32;
+  }
   switch (nt) {
     case 512: launch_nt<512, 32>(p, g, st); break;
     case 384: launch_nt<384, 32>(p, g, st); break;

@@ -54,3 +54,14 @@ def test_every_block_size_gives_the_oracles_bits(cuda, n):
 def test_odd_layer_shapes_give_the_oracles_bits(cuda, net):
     _check(_net(**net), 67, 5, 19, clamp=False, kahan=False)
     _check(_net(**net), 419, 53, 2)
+
+
+@pytest.mark.parametrize("net", [dict(levels=24, features=8, aux=13, op=(33, 7, 33), cn=(33, 7)),
+                                 dict(levels=20, features=8, op=(36, 7, 53), cn=(36, 7)),
+                                 dict(levels=27, features=6, aux=19, op=(36, 7, 40), cn=(40, 7))])
+def test_largest_networks_run_with_fewer_wavelets_at_a_time(cuda, net):
+    # accepted by the unpadded limit; their padded weight rows leave room for 8, 8 and 2 wavelets'
+    # embedding rows beside 32 pixels
+    cfg = _net(**net)
+    cfg["vtx_enc"]["per_level_scale"] = 1.2
+    _check(cfg, 67, 5, 19)
