@@ -29,7 +29,7 @@ __device__ __forceinline__ void uv_to_dir(int f, float uc, float vc, float& x, f
   }
 }
 
-__global__ void env_rotate_kernel(const float* __restrict__ src, int S, Rot R, float* __restrict__ dst) {
+__global__ void env_rotate_kernel(const float* src, int S, Rot R, float* dst) {
   let_next_start();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long SS = (long long)S * S;
@@ -68,9 +68,10 @@ __global__ void env_rotate_kernel(const float* __restrict__ src, int S, Rot R, f
   stream_wait(src, dst);
   const float* s = src + (((long long)sf * S + row) * S + col) * 3;
   float* d = dst + t * 3;
-  d[0] = s[0];
-  d[1] = s[1];
-  d[2] = s[2];
+  const float v0 = ld_stream(s), v1 = ld_stream(s + 1), v2 = ld_stream(s + 2);
+  d[0] = v0;
+  d[1] = v1;
+  d[2] = v2;
 }
 
 }  // namespace

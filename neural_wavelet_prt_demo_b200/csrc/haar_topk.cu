@@ -252,14 +252,14 @@ __device__ __forceinline__ int flat_in_face(int tid, int u) {
 // its 2x2 quad, a level-2 detail from the four quads' LL values.  The batched kernel keeps no copy
 // of these coefficients; it recomputes the K winners' instead.
 template <int S>
-__device__ __forceinline__ float block_coef(const float* __restrict__ src, int tid, int u, int c) {
+__device__ __forceinline__ float block_coef(const float* src, int tid, int u, int c) {
   using F = FaceGeom<S>;
   const int bj = morton_even(tid), bi = morton_even(tid >> 1);
   const float* blk = src + ((size_t)(F::B * bi) * S + F::B * bj) * 3 + c;
   const int q = u / 3, band = u % 3;
   auto quad = [&](int qi, int qj, float& a, float& hl, float& lh, float& hh) {
     const float* p0 = blk + ((size_t)(2 * qi) * S + 2 * qj) * 3;
-    haar4(__ldg(p0), __ldg(p0 + 3), __ldg(p0 + S * 3), __ldg(p0 + S * 3 + 3), a, hl, lh, hh);
+    haar4(ld_stream(p0), ld_stream(p0 + 3), ld_stream(p0 + S * 3), ld_stream(p0 + S * 3 + 3), a, hl, lh, hh);
   };
   float a, hl, lh, hh;
   if (q < 4) {
@@ -278,7 +278,7 @@ __device__ __forceinline__ float block_coef(const float* __restrict__ src, int t
 // its NR detail coefficients, ll: the block's LL value), with the same operations in the same
 // order as haar_face_in_registers.
 template <int S>
-__device__ __forceinline__ void block_load(const float* __restrict__ src, int tid,
+__device__ __forceinline__ void block_load(const float* src, int tid,
                                            float (&px)[FaceGeom<S>::B][FaceGeom<S>::B][3]) {
   using F = FaceGeom<S>;
   constexpr int B = F::B;
@@ -292,7 +292,7 @@ __device__ __forceinline__ void block_load(const float* __restrict__ src, int ti
         const float4* row = reinterpret_cast<const float4*>(blk + (size_t)r * S * 3);
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-          const float4 v = __ldg(row + q);
+          const float4 v = ld_stream(row + q);
           const float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
           for (int k = 0; k < 4; ++k) px[r][(4 * q + k) / 3][(4 * q + k) % 3] = e[k];
@@ -302,13 +302,13 @@ __device__ __forceinline__ void block_load(const float* __restrict__ src, int ti
 #pragma unroll
       for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int q = 0; q < 12; ++q) px[r][q / 3][q % 3] = __ldg(blk + (size_t)r * S * 3 + q);
+        for (int q = 0; q < 12; ++q) px[r][q / 3][q % 3] = ld_stream(blk + (size_t)r * S * 3 + q);
     }
   } else {
 #pragma unroll
     for (int r = 0; r < B; ++r)
 #pragma unroll
-      for (int q = 0; q < 3 * B; ++q) px[r][q / 3][q % 3] = __ldg(blk + (size_t)r * S * 3 + q);
+      for (int q = 0; q < 3 * B; ++q) px[r][q / 3][q % 3] = ld_stream(blk + (size_t)r * S * 3 + q);
   }
 }
 
@@ -370,7 +370,7 @@ __device__ __forceinline__ void block_levels(const float (&px)[FaceGeom<S>::B][F
 // result (levels >= 3 and the DC term) lands in `upper` [G*G][3]; `llg` is [16][3] staging.
 // Ends with a block barrier, after which `upper` is complete.
 template <int S>
-__device__ __forceinline__ void haar_face_in_registers(const float* __restrict__ src, int tid,
+__device__ __forceinline__ void haar_face_in_registers(const float* src, int tid,
                                                        float (&co)[FaceGeom<S>::NR > 0 ? FaceGeom<S>::NR : 1][3],
                                                        float* upper, float* llg) {
   using F = FaceGeom<S>;
@@ -426,8 +426,8 @@ __device__ __forceinline__ void haar_face_in_registers(const float* __restrict__
 template <int S>
 // Two CTAs per SM at most: the bound leaves the transform its registers (three per SM spilled).
 __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
-    haar_topk_kernel(const float* __restrict__ faces, int K, int32_t* __restrict__ idx_out,
-                     float* __restrict__ st_out) {
+    haar_topk_kernel(const float* faces, int K, int32_t* idx_out,
+                     float* st_out) {
   using F = FaceGeom<S>;
   constexpr int T = F::T, SS = F::SS, NR = F::NR;
   constexpr int NW = (SS + 31) / 32;
@@ -768,7 +768,7 @@ __host__ __device__ inline size_t batch_smem_layout(int S, int K, char* base, Ba
 // The keys of the NR detail coefficients of texel block tid (0 for u == NR and for a thread without one)
 // and its block's LL value, with the operations of block_levels, two texel rows at a time.
 template <int S>
-__device__ __forceinline__ void face_keys(const float* __restrict__ src, bool owner, int tid,
+__device__ __forceinline__ void face_keys(const float* src, bool owner, int tid,
                                           uint32_t (&k)[FaceGeom<S>::NK], float (&ll)[3]) {
   using F = FaceGeom<S>;
   constexpr int B = F::B;
@@ -780,7 +780,7 @@ __device__ __forceinline__ void face_keys(const float* __restrict__ src, bool ow
   const float* blk = src + ((size_t)(B * bi) * S + B * bj) * 3;
   if constexpr (B == 1) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) ll[c] = __ldg(blk + c);
+    for (int c = 0; c < 3; ++c) ll[c] = ld_stream(blk + c);
   } else {
     float l1[B == 4 ? 4 : 1][3];
     const bool vec = B == 4 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
@@ -793,7 +793,7 @@ __device__ __forceinline__ void face_keys(const float* __restrict__ src, bool ow
         if (vec) {
 #pragma unroll
           for (int q = 0; q < B * 3 / 4; ++q) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(row) + q);
+            const float4 v = ld_stream(reinterpret_cast<const float4*>(row) + q);
             px[r][4 * q] = v.x;
             px[r][4 * q + 1] = v.y;
             px[r][4 * q + 2] = v.z;
@@ -801,7 +801,7 @@ __device__ __forceinline__ void face_keys(const float* __restrict__ src, bool ow
           }
         } else {
 #pragma unroll
-          for (int q = 0; q < B * 3; ++q) px[r][q] = __ldg(row + q);
+          for (int q = 0; q < B * 3; ++q) px[r][q] = ld_stream(row + q);
         }
       }
 #pragma unroll
@@ -956,7 +956,7 @@ struct KeyList {
 
 // Lists a map's keys once more, those from lo_key up (counts untouched).
 template <int S>
-__device__ __noinline__ void list_again(const float* __restrict__ map, uint32_t lo_key, int K) {
+__device__ __noinline__ void list_again(const float* map, uint32_t lo_key, int K) {
   using F = FaceGeom<S>;
   extern __shared__ __align__(16) char smem_raw[];
   BatchSmem sm;
@@ -985,7 +985,7 @@ __device__ __noinline__ void list_again(const float* __restrict__ map, uint32_t 
 // The K winners of a map whose lists overflowed, into gkey / gid: a 4-pass 8-bit radix select that
 // recomputes the keys in each pass, then ties at the threshold in flat-index order by a bitmap.
 template <int S>
-__device__ __noinline__ void general_select(const float* __restrict__ map, int K) {
+__device__ __noinline__ void general_select(const float* map, int K) {
   using F = FaceGeom<S>;
   extern __shared__ __align__(16) char smem_raw[];
   BatchSmem sm;
@@ -1067,8 +1067,8 @@ __device__ __noinline__ void general_select(const float* __restrict__ map, int K
 
 template <int S>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
-    haar_topk_batch_kernel(const float* __restrict__ faces, int n_env, int K, int32_t* __restrict__ idx_out,
-                           float* __restrict__ st_out) {
+    haar_topk_batch_kernel(const float* faces, int n_env, int K, int32_t* idx_out,
+                           float* st_out) {
   using F = FaceGeom<S>;
   constexpr int T = F::T, SS = F::SS, NR = F::NR, NK = F::NK, G = F::G;
   constexpr int NL = G >= 8 ? G / 4 : 1;  // side of the LL grid left after levels 3-4

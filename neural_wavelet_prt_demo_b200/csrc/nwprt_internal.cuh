@@ -7,6 +7,7 @@
 
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/nwprt.h"
@@ -397,13 +398,39 @@ __device__ __forceinline__ void fence_barrier_init() {
 }
 
 // The kernels before this one in the stream have completed and their writes are visible.  Every
-// thread that touches global memory calls it; pointers pass through it so that no load of what they
-// point to, read-only ones included, moves above it.
+// thread that touches global memory calls it, and reads what earlier work in the stream may have
+// written by ld_stream; pointers pass through it so that no other access to what they point to moves
+// above it.
 template <class... PTR>
 __device__ __forceinline__ void stream_wait(PTR&... ptrs) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   auto opaque = [](auto& p) { asm volatile("" : "+l"(p)::"memory"); };
   (opaque(ptrs), ...);
+}
+
+// A load of memory that an earlier kernel in the stream may write while this one, launched by
+// launch_overlapped, is already resident.  The non-coherent load (__ldg, or what a const __restrict__
+// pointer lets the compiler make of a plain one) is for memory that stays read-only while the kernel
+// lives, and stream_wait does not order it: a line cached before may be served after.  This is the
+// ordinary load, and stays below every stream_wait above it.
+template <class T>
+__device__ __forceinline__ T ld_stream(const T* p) {
+  T v;
+  if constexpr (std::is_same<T, float>::value) {
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  } else if constexpr (std::is_same<T, float4>::value) {
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  } else if constexpr (std::is_same<T, uint4>::value) {
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  } else if constexpr (std::is_same<T, int32_t>::value) {
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  } else {
+    static_assert(std::is_same<T, uint8_t>::value, "ld_stream: no form for this type");
+    uint32_t b;
+    asm volatile("ld.global.u8 %0, [%1];" : "=r"(b) : "l"(p));
+    v = (uint8_t)b;
+  }
+  return v;
 }
 
 // The next kernel in the stream may start once every block has called this (or ended): it gets

@@ -16,16 +16,15 @@
 namespace nwprt {
 namespace {
 
-__global__ void pack_gbuffer_kernel(int64_t n, const float4* __restrict__ pos,
-                                    const float4* __restrict__ nrm, const float4* __restrict__ refl,
-                                    const float* __restrict__ rough, const float4* __restrict__ kd,
-                                    const float4* __restrict__ ks, float rgh_den,
-                                    float4* __restrict__ out) {
+__global__ void pack_gbuffer_kernel(int64_t n, const float4* pos, const float4* nrm, const float4* refl,
+                                    const float* rough, const float4* kd, const float4* ks, float rgh_den,
+                                    float4* out) {
   let_next_start();
   stream_wait(pos, nrm, refl, rough, kd, ks, out);
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
-  const float4 a = pos[p], b = nrm[p], c = refl[p], d = kd[p], e = ks[p];
+  const float4 a = ld_stream(pos + p), b = ld_stream(nrm + p), c = ld_stream(refl + p), d = ld_stream(kd + p),
+               e = ld_stream(ks + p);
   const float r = logf_series(fmaf(25.f, rough[p], 1.f)) * rgh_den;
   out[p * 4 + 0] = make_float4(a.x, a.y, a.z, b.x);
   out[p * 4 + 1] = make_float4(b.y, b.z, c.x, c.y);
@@ -34,16 +33,15 @@ __global__ void pack_gbuffer_kernel(int64_t n, const float4* __restrict__ pos,
 }
 
 // One thread per feature pair (k, 2i..2i+1): both FP32 values, and (out_h) their BF16 pair.
-__global__ void gather_embedding_kernel(const float* __restrict__ emb, int D, int n_coeffs,
-                                        const int32_t* __restrict__ idx, int K,
-                                        float* __restrict__ out, uint32_t* __restrict__ out_h, uint32_t* err) {
+__global__ void gather_embedding_kernel(const float* __restrict__ emb, int D, int n_coeffs, const int32_t* idx,
+                                        int K, float* out, uint32_t* out_h, uint32_t* err) {
   let_next_start();
   stream_wait(emb, idx, out, out_h);
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int H = D / 2;
   if (t >= (int64_t)K * H) return;
   const int k = (int)(t / H), d = 2 * (int)(t - (int64_t)k * H);
-  const int32_t j = idx[k];
+  const int32_t j = ld_stream(idx + k);
   float v0 = 0.f, v1 = 0.f;
   if (j >= 0 && j < n_coeffs) {
     v0 = emb[(int64_t)d * n_coeffs + j];

@@ -504,15 +504,14 @@ struct EncRow {
 // recording max |hash(p) * E_k| in amax[0].  FP8: from the FP32 row, scaled by cp_scale and
 // rounded to E4M3, zero-padded to K = 32.
 template <int DMAX, int MODE>
-__device__ __forceinline__ void store_cp(const EncRow<DMAX>& enc, const float* __restrict__ ek,
-                                         const uint32_t* __restrict__ eh, uint32_t a_taddr, float cp_scale,
-                                         uint32_t* amax) {
+__device__ __forceinline__ void store_cp(const EncRow<DMAX>& enc, const float* ek, const uint32_t* eh, uint32_t a_taddr,
+                                         float cp_scale, uint32_t* amax) {
   constexpr int NW = MODE == kTcFp8 ? 8 : DMAX / 2;
   uint32_t cp[NW];
   if constexpr (MODE == kTcBf16) {
 #pragma unroll
     for (int c = 0; c < DMAX / 8; ++c) {
-      const uint4 e = __ldg(reinterpret_cast<const uint4*>(eh) + c);
+      const uint4 e = ld_stream(reinterpret_cast<const uint4*>(eh) + c);
       const uint4 h = enc.get(c);
       const uint32_t ev[4] = {e.x, e.y, e.z, e.w}, hv[4] = {h.x, h.y, h.z, h.w};
 #pragma unroll
@@ -525,8 +524,8 @@ __device__ __forceinline__ void store_cp(const EncRow<DMAX>& enc, const float* _
   float m = 0.f;
 #pragma unroll
   for (int c = 0; c < DMAX / 8; ++c) {
-    const float4 e0 = __ldg(reinterpret_cast<const float4*>(ek + c * 8));
-    const float4 e1 = __ldg(reinterpret_cast<const float4*>(ek + c * 8 + 4));
+    const float4 e0 = ld_stream(reinterpret_cast<const float4*>(ek + c * 8));
+    const float4 e1 = ld_stream(reinterpret_cast<const float4*>(ek + c * 8 + 4));
     const uint4 h = enc.get(c);
     const uint32_t h0 = h.x, h1 = h.y, h2 = h.z, h3 = h.w;
     const float x0 = __fmul_rn(bf16_lo(h0), e0.x), x1 = __fmul_rn(bf16_hi(h0), e0.y);
@@ -830,7 +829,7 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
     const EncRow<DMAX> enc_s(encs + (shared_tile() ? 0 : g) * (DMAX / 2) * kTile, row);
     {
       const float4* pr = reinterpret_cast<const float4*>(J.packed) + (valid ? px : J.n_px - 1) * 4;
-      const float4 r0 = __ldg(pr);
+      const float4 r0 = ld_stream(pr);
       auto put = [&](int l, uint32_t v) { enc_s.put_pair(l, valid ? v : 0u); };
       if (shared_tile()) {
         hash_encode_pairs(p.hl, p.hash, r0.x, r0.y, r0.z, g, DMAX / 2, kNWG, put);
@@ -842,7 +841,7 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
       }
       if (valid) {
         // aux operand: the 13 remapped G-buffer values followed by ones
-        const float4 r1 = __ldg(pr + 1), r2 = __ldg(pr + 2), r3 = __ldg(pr + 3);
+        const float4 r1 = ld_stream(pr + 1), r2 = ld_stream(pr + 2), r3 = ld_stream(pr + 3);
         st_shared_v4(aux_row, pack_bf16(r0.w, r1.x), pack_bf16(r1.y, r1.z), pack_bf16(r1.w, r2.x),
                      pack_bf16(r2.y, r2.z));
         st_shared_v4(aux_row + 128u, pack_bf16(r2.w, r3.x), pack_bf16(r3.y, r3.z), pack_bf16(r3.w, 1.f),
@@ -883,7 +882,7 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
         L0 = Lk.x; L1 = Lk.y; L2 = Lk.z;
       } else {
         const float* Lk = J.strength + (size_t)(k_begin_now() + k) * 3;
-        L0 = __ldg(Lk + 0); L1 = __ldg(Lk + 1); L2 = __ldg(Lk + 2);
+        L0 = ld_stream(Lk + 0); L1 = ld_stream(Lk + 1); L2 = ld_stream(Lk + 2);
       }
       float u0 = __fmul_rn(L0, t0);
       float u1 = __fmul_rn(L1, t1);
@@ -1044,9 +1043,9 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
     if (ok && (!shared_tile() || g == 0)) {
       const long long px = J.px_begin + (t - J.tile_begin) * kTile + row;
       if (px < J.n_px) {
-        const float4 ind = J.flag[px] ? make_float4(my_sums[0], my_sums[kTile], my_sums[2 * kTile], 1.f)
+        const float4 ind = ld_stream(J.flag + px) ? make_float4(my_sums[0], my_sums[kTile], my_sums[2 * kTile], 1.f)
                                       : make_float4(0.f, 0.f, 0.f, 1.f);
-        const float4 dl = __ldg(reinterpret_cast<const float4*>(J.direct) + px);
+        const float4 dl = ld_stream(reinterpret_cast<const float4*>(J.direct) + px);
         reinterpret_cast<float4*>(J.indirect)[px] = ind;
         reinterpret_cast<float4*>(J.with_direct)[px] =
             make_float4(__fadd_rn(ind.x, dl.x), __fadd_rn(ind.y, dl.y), __fadd_rn(ind.z, dl.z), 1.f);

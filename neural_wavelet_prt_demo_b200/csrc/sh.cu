@@ -104,8 +104,8 @@ constexpr int kProjGroup = kNc / 3;                       // 27 threads cover th
 constexpr int kProjSlices = kProjThreads / kProjGroup;    // 9
 constexpr size_t kProjSmem = sizeof(float) * (4 * kProjThreads + kNc * kProjPad);
 
-__global__ void __launch_bounds__(kProjThreads) sh_project_partial(const float* __restrict__ faces, int S,
-                                                                   int n_chunks, float* __restrict__ part) {
+__global__ void __launch_bounds__(kProjThreads) sh_project_partial(const float* faces, int S, int n_chunks,
+                                                                   float* part) {
   extern __shared__ __align__(16) float sm[];
   float4* sF = reinterpret_cast<float4*>(sm);  // [256]            texel radiance
   float* sY = sm + 4 * kProjThreads;           // [81][kProjPad]   Y_k * dA
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kProjThreads) sh_project_partial(const float* 
       const int rem = (int)(t - (long long)f * SS);
       const int r = rem / S, c = rem - r * S;
       const float* tx = faces + t * 3;
-      sF[tid] = make_float4(tx[0], tx[1], tx[2], 0.f);
+      sF[tid] = make_float4(ld_stream(tx), ld_stream(tx + 1), ld_stream(tx + 2), 0.f);
       const float uc = 2.f * (c + 0.5f) / S - 1.f, vc = 2.f * (r + 0.5f) / S - 1.f;
       float x, y, z;
       switch (f) {
@@ -179,8 +179,7 @@ __global__ void __launch_bounds__(kProjThreads) sh_project_partial(const float* 
 
 // L = the sum of the blocks' partial sums: a block takes 32 of the 243 sums, its warp w the
 // partial sums w, w + 32, ..., and warp 0 adds the warps' results in order.
-__global__ void __launch_bounds__(1024) sh_project_reduce(const float* __restrict__ part, int n_blocks,
-                                                          float* __restrict__ L) {
+__global__ void __launch_bounds__(1024) sh_project_reduce(const float* part, int n_blocks, float* L) {
   __shared__ float sums[32][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int o = blockIdx.x * 32 + lane;
@@ -188,7 +187,7 @@ __global__ void __launch_bounds__(1024) sh_project_reduce(const float* __restric
   stream_wait(part, L);
   if (o < kNc * 3)
 #pragma unroll 8
-    for (int b = warp; b < n_blocks; b += 32) acc += part[(size_t)b * (kNc * 3) + o];
+    for (int b = warp; b < n_blocks; b += 32) acc += ld_stream(part + (size_t)b * (kNc * 3) + o);
   sums[warp][lane] = acc;
   __syncthreads();
   if (warp == 0 && o < kNc * 3) {

@@ -53,14 +53,18 @@ __device__ __forceinline__ uint32_t lookup(const float* t, float x) {
   return (uint32_t)j + (t[j + 1] <= x ? 1u : 0u);
 }
 
-// HBM-bound.  A shared-memory lookup of a pseudo-random threshold meets a 3-way bank conflict, so
-// one lookup per channel instead of three to four, and the table's load off the constant bank, took
-// 16 1080p frames from 160 to 103 us (6,440 GB/s) and one 2559 x 1439 frame from 23.6 to 14.2 us.
-// One pixel per thread and iteration on 8 blocks per SM (every thread slot): 2 or 4 pixels measured
-// 16.8 and 17.4 us on that frame, 64 blocks per SM 18.1 us (100 us on the 16 frames).
+// Pixels per thread and iteration.
+constexpr int kInFlight = 3;
+
+// HBM-bound.  A shared-memory lookup of a pseudo-random threshold meets a 3-way bank conflict, so one
+// lookup per channel instead of three to four, and the table's load off the constant bank, took 16
+// 1080p frames from 160 to 103 us and one 2559 x 1439 frame from 23.6 to 14.2 us.  8 blocks per SM
+// (every thread slot) a whole grid apart: 64 per SM measured 18.1 us on that frame.  An ordinary load
+// does not move above a store, so an iteration's loads are written before its first store: 16 frames,
+// that frame and a 1080p one take 101.4 (6,540 GB/s), 13.1 and 8.5 us with three of them (two: 103.8,
+// 13.4 and 8.7; four: 100.8, 13.0 and 9.1; one at a time: 119, 14.4 and 9.0).
 __global__ void __launch_bounds__(256) tonemap_srgb_kernel(const __grid_constant__ SrgbTable T,
-                                                           const float4* __restrict__ src, int64_t n,
-                                                           uint32_t* __restrict__ dst) {
+                                                           const float4* src, int64_t n, uint32_t* dst) {
   __shared__ float t[256];
   const float* table = T.t;
   asm volatile("" : "+l"(table));  // one coalesced load, not 32 constant-bank reads per warp
@@ -68,10 +72,22 @@ __global__ void __launch_bounds__(256) tonemap_srgb_kernel(const __grid_constant
   __syncthreads();
   let_next_start();
   stream_wait(src, dst);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float4 v = __ldg(src + i);
-    dst[i] = lookup(t, v.x) | (lookup(t, v.y) << 8) | (lookup(t, v.z) << 16) | (255u << 24);
+  // kInFlight loads are issued before the first store, above which an ordinary load does not move
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  auto put = [&](int64_t at, const float4& v) {
+    dst[at] = lookup(t, v.x) | (lookup(t, v.y) << 8) | (lookup(t, v.z) << 16) | (255u << 24);
+  };
+#pragma unroll 1
+  for (; i + (kInFlight - 1) * step < n; i += kInFlight * step) {
+    float4 v[kInFlight];
+#pragma unroll
+    for (int k = 0; k < kInFlight; ++k) v[k] = ld_stream(src + i + k * step);
+#pragma unroll
+    for (int k = 0; k < kInFlight; ++k) put(i + k * step, v[k]);
   }
+#pragma unroll 1
+  for (; i < n; i += step) put(i, ld_stream(src + i));
 }
 
 }  // namespace
