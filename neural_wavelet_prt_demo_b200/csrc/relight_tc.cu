@@ -574,7 +574,10 @@ __device__ __forceinline__ void store_cp_smem(const EncRow<DMAX>& enc, const uin
 }
 
 // Adds a chunk's channel sums s (with their Kahan compensations c: the sum is s - c) to a pixel's
-// running ones at tot, [6][kTile]: three sums, three compensations.  init: tot's first chunk.
+// running ones at tot, [6][kTile]: three sums, three compensations.  init: tot's first chunk.  ENDS:
+// it may be tot's last chunk, whose last term may be the sum's only infinite one: its compensation
+// then is not a number, and stays out.  (More terms after an infinite one give NaN, Kahan's way.)
+template <bool ENDS>
 __device__ __forceinline__ void add_chunk(float* tot, bool init, int kahan, float s0, float s1, float s2, float c0,
                                           float c1, float c2) {
   const float s[3] = {s0, s1, s2}, c[3] = {c0, c1, c2};
@@ -588,7 +591,7 @@ __device__ __forceinline__ void add_chunk(float* tot, bool init, int kahan, floa
         float y = __fsub_rn(s[i], C), z = __fadd_rn(S, y);
         C = __fsub_rn(__fsub_rn(z, S), y);
         S = z;
-        y = __fsub_rn(-c[i], C);
+        y = ENDS && fabsf(S) == INFINITY ? 0.f : __fsub_rn(-c[i], C);
         z = __fadd_rn(S, y);
         C = __fsub_rn(__fsub_rn(z, S), y);
         S = z;
@@ -870,7 +873,7 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
     float* my_sums = sums + g * 6 * kTile + row;
     // the chunk's sums join the tile's
     auto flush = [&] {
-      add_chunk(my_sums, flush_at == chunk(), p.kahan, s0, s1, s2, c0, c1, c2);
+      add_chunk<false>(my_sums, flush_at == chunk(), p.kahan, s0, s1, s2, c0, c1, c2);
       s0 = s1 = s2 = c0 = c1 = c2 = 0.f;
       flush_at += chunk();
     };
@@ -1030,15 +1033,16 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
     t = tile_now();
     if (shared_tile()) {
       // the chunks' sums meet in warpgroup 0, in order
-      add_chunk(my_sums, true, p.kahan, s0, s1, s2, c0, c1, c2);
+      add_chunk<true>(my_sums, true, p.kahan, s0, s1, s2, c0, c1, c2);
       ok = __syncthreads_and(ok);
       if (g == 0)
         for (int j = 1; j * chunk() < J.K; ++j) {
           const float* o = my_sums + j * 6 * kTile;
-          add_chunk(my_sums, false, p.kahan, o[0], o[kTile], o[2 * kTile], o[3 * kTile], o[4 * kTile], o[5 * kTile]);
+          add_chunk<true>(my_sums, false, p.kahan, o[0], o[kTile], o[2 * kTile], o[3 * kTile], o[4 * kTile],
+                          o[5 * kTile]);
         }
     } else if (flush_at - chunk() < K) {
-      add_chunk(my_sums, flush_at == chunk(), p.kahan, s0, s1, s2, c0, c1, c2);  // the last, shorter chunk
+      add_chunk<true>(my_sums, flush_at == chunk(), p.kahan, s0, s1, s2, c0, c1, c2);  // the last, shorter chunk
     }
     if (ok && (!shared_tile() || g == 0)) {
       const long long px = J.px_begin + (t - J.tile_begin) * kTile + row;

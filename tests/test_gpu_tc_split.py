@@ -85,3 +85,28 @@ def test_split_without_the_tensor_core_output_layer(cuda, net, precision, K):
     for part in out[1:]:
         assert np.array_equal(part.view(np.uint32), out[0][:len(part)].view(np.uint32))
     e.close()
+
+
+@pytest.mark.parametrize("w,h", [(67, 5), (1021, 97)])
+@pytest.mark.parametrize("K", [1, 5, 13])
+def test_infinite_last_term_gives_infinity(cuda, w, h, K):
+    # the compensation of a chunk that ends in an infinite term is not a number and must stay out of
+    # the sum: infinity (or, where T_k < 0 is clamped, the finite rest), as without compensation
+    from neural_wavelet_prt_demo_b200 import engine as eng
+    case = make_case(netconfig.CONFIG_SMALL, w, h, K, seed=K, hash_scale=0.5)
+    strength = case.strength.copy()
+    strength[-1] = np.inf
+    e = eng.RenderEngine(case.cfg)
+    e.loadWeights(case.weights)
+    env = e.addEnvironmentMap(eng.EnvironmentMap(top_coefficients=case.idx, top_strength=strength))
+    fr = eng.FullFrame.from_gbuffer(case.gbuf)
+    e.setFrame(0, fr)
+    e.TCNNPass_p1(0)
+    out = []
+    for kahan in (True, False):
+        e.TCNNPass_p2(env, 0, eng.RenderConfig(precision="bf16", kahan=kahan))
+        e.TCNNSync()
+        out.append(fr.fbPredictedIndirect.cpu().numpy()[:, :3])
+    assert not np.isnan(out[0]).any()
+    assert np.isinf(out[0]).any() and np.array_equal(np.isinf(out[0]), np.isinf(out[1]))
+    e.close()
