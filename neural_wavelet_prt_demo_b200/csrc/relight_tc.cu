@@ -858,7 +858,7 @@ __global__ void __launch_bounds__(kThreads, 1) relight_tc_kernel(const __grid_co
     ok = wait_bounded(&bars->wload, 0, p.err) && ok;
     if (shared_tile()) ok = __syncthreads_and(ok);  // the tile's features are complete
     float s0 = 0.f, s1 = 0.f, s2 = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f;
-    int flush_at = shared_tile() ? 0 : chunk();  // the wavelet that the next chunk starts with (0: never)
+    int flush_at = shared_tile() ? -1 : chunk();  // the wavelet that the next chunk starts with (-1: no next one)
     if (K > 0) {
       const int kb = k_begin();
       store_cp<DMAX, MODE>(enc_s, J.emb_k + (size_t)kb * p.enc_dims, J.emb_h + (size_t)kb * (p.enc_dims / 2), a_taddr,
