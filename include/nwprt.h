@@ -244,6 +244,10 @@ NWPRT_API nwprt_status nwprt_tonemap_srgb(const float* src, int64_t n_px, uint32
  * out: [V][3]; n = (degree + 1)^2 <= 81.  All device memory. */
 NWPRT_API nwprt_status nwprt_sh_vertex_radiance(const float* T, const float* brdf_sh, const float* L,
                                                 int64_t n_vertices, int n_coeffs, float* out, void* stream);
+/* Diagnostics: nwprt_sh_vertex_radiance with every wait for a matrix's copy into shared memory giving
+ * up at once.  A warp whose wait runs out reads its matrices where they are: the results are the same. */
+NWPRT_API nwprt_status nwprt_selftest_sh_vertex(const float* T, const float* brdf_sh, const float* L,
+                                                int64_t n_vertices, int n_coeffs, float* out, void* stream);
 /* Pixel colours from their triangle's vertex colours (devicePrograms.cu:488-490):
  * out[p] = ((1 - u - v) c[i0] + u c[i1] + v c[i2], 1), evaluated as
  * fma(v, c2, fma(u, c1, (1 - u - v) c0)).  tri: [P][3] int32 vertex indices, uv: [P][2]

@@ -752,7 +752,16 @@ nwprt_status nwprt_tonemap_srgb(const float* src, int64_t n_px, uint32_t* dst, v
 
 nwprt_status nwprt_sh_vertex_radiance(const float* T, const float* brdf_sh, const float* L, int64_t n_vertices,
                                       int n_coeffs, float* out, void* stream) {
-  return guarded(nullptr, [&] { launch_sh_vertex(T, brdf_sh, L, n_vertices, n_coeffs, out, (cudaStream_t)stream); });
+  return guarded(nullptr, [&] {
+    launch_sh_vertex(T, brdf_sh, L, n_vertices, n_coeffs, out, kWaitPolls, (cudaStream_t)stream);
+  });
+}
+
+nwprt_status nwprt_selftest_sh_vertex(const float* T, const float* brdf_sh, const float* L, int64_t n_vertices,
+                                      int n_coeffs, float* out, void* stream) {
+  return guarded(nullptr, [&] {
+    launch_sh_vertex(T, brdf_sh, L, n_vertices, n_coeffs, out, 0, (cudaStream_t)stream);
+  });
 }
 
 nwprt_status nwprt_sh_interpolate(nwprt_ctx* ctx, const float* vertex_rgb, int64_t n_vertices, const int32_t* tri,

@@ -176,7 +176,7 @@ void launch_tonemap_srgb(const float* src, int64_t n, uint32_t* dst, cudaStream_
 
 // sh_vertex.cu
 void launch_sh_vertex(const float* T, const float* brdf, const float* L, int64_t V, int n, float* out,
-                      cudaStream_t st);
+                      uint32_t polls, cudaStream_t st);
 void launch_sh_interpolate(const float* vc, int64_t V, const int32_t* tri, const float* uv, int64_t P, float* out,
                            uint32_t* err, cudaStream_t st);
 
@@ -255,10 +255,12 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+constexpr uint32_t kWaitPolls = 1u << 26;
+
 // Bounded mbarrier wait.  Returns false (and records kDevWaitTimeout) when the
 // phase did not complete within `limit` polls; callers then abandon their work.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t* err,
-                                          uint32_t limit = (1u << 26)) {
+                                          uint32_t limit = kWaitPolls) {
   const uint32_t a = smem_u32(bar);
   for (uint32_t it = 0; it < limit; ++it) {
     uint32_t done;

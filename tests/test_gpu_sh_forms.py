@@ -24,3 +24,19 @@ def test_sh_vertex_forms_bit_exact(cuda, n, shift):
     Td.copy_(torch.from_numpy(T))
     got = eng.sh_vertex_radiance(Td, *(torch.from_numpy(a).to(cuda) for a in (brdf, L))).cpu().numpy()
     assert np.array_equal(got.view(np.uint32), O.sh_vertex_radiance(T, brdf, L).view(np.uint32))
+
+
+@pytest.mark.parametrize("n", [1, 9, 33, 36, 62, 64, 81])
+def test_sh_vertex_waits_that_run_out_lose_nothing(cuda, n):
+    # the call has no status for a wait that gave up, so the results have to be right all the same
+    import torch
+    from neural_wavelet_prt_demo_b200 import _lib
+    V = 2501  # more than the blocks' warps: a warp goes on after the wait that ran out
+    T, brdf, _, _ = synth.make_sh_mesh(V, 1, 81, seed=n)
+    T, brdf = T[:, :n, :n].copy(), brdf[:, :n].copy()
+    L = synth.make_sh_transport(3, 81, seed=5).T[:n].copy()
+    Td, bd, Ld = (torch.from_numpy(a).to(cuda) for a in (T, brdf, L))
+    out = torch.full((V, 3), float("nan"), device=cuda)
+    _lib.check(_lib.lib().nwprt_selftest_sh_vertex(Td.data_ptr(), bd.data_ptr(), Ld.data_ptr(), V, n, out.data_ptr(),
+                                                   torch.cuda.current_stream().cuda_stream))
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), O.sh_vertex_radiance(T, brdf, L).view(np.uint32))
