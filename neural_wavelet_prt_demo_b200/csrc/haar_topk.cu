@@ -680,11 +680,16 @@ __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
 // SM beat the cluster's one sixth of a map each, and no step crosses an SM.
 //
 // Few of a map's coefficients can be among its K largest, so their keys are not kept.  The CTA
-// transforms the six faces one after another, histogramming the first face's keys by their top 11
-// bits (the exponent and 3 bits of the fraction).  The K-th largest key seen so far is a lower bound
+// transforms the map in six steps of a face's size, histogramming the first step's keys by their top
+// 11 bits (the exponent and 3 bits of the fraction).  The K-th largest key seen so far is a lower bound
 // of the K-th largest of all: a warp lists only its keys from that one's bin up, counts what it
-// lists, and looks the bound up again at the third face, before it lists much of one (a face
-// brighter than the ones before), and from face to face once the list is crowded.
+// lists, and looks the bound up again at the third step, before it lists much of one (brighter than
+// what came before), and from step to step once the list is crowded.  A step of a 64 x 64 map is an
+// eighth of a face per warp, of another face each, so that the first one sees all of them: face by
+// face, maps whose faces grow brighter listed too much and were read twice (each ten times brighter
+// than the one before: 173 us, now 95; twice: 132, now 101).  No single copy can fetch the next step
+// ahead then, which four CTAs per SM do without (line by line: 110.7 against 107.2 us; three per SM,
+// K = 1024: 203 -> 212).  Taking the faces by a sample of their detail, the largest first: 112.2 us.
 // No barrier guards the look-up: counts still missing only lower the bound.  When the upper levels
 // are done, one block scan over the bins gives the last winner's bin, the listed keys from it up go
 // to their bin's part of a second list, and each is ranked among its own bin's keys only.  Keys
@@ -704,8 +709,7 @@ __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
 // 6 K + 768 keys instead of 5 K + 512 took one step of it: 110 -> 117 us).  1,024 maps, K = 300:
 // 132 us -> 107 (2,870 GB/s) with all keys kept in shared memory, three scans of them and two CTAs
 // per SM before; K = 64 109 -> 86, K = 1024 229 -> 202; S = 32 102 -> 50; S = 16, K = 64 67 -> 19;
-// maps of few lights on black 269 -> 84.  Each face ten times brighter than the one before is the
-// bad case: 121 -> 174.  Of these, one prefix sum per list instead of a ballot per key and writing the
+// maps of few lights on black 269 -> 84.  Of these, one prefix sum per list instead of a ballot per key and writing the
 // level-2 winners apart give 109.4 -> 107.1 (K = 64 86.4 -> 85.9, K = 1024 208.8 -> 202.3).
 
 constexpr int kBins = 2048;       // of keys by bits 30..20
@@ -1091,10 +1095,11 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     __syncthreads();
     KeyList list{sm, K, cap, lane};
     for (int f0 = 0; f0 < 6; f0 += F::FPI) {
-      const int f = f0 + fi;
+      // one face at a time: each warp its part of another one (see above)
+      const int f = F::FPI == 1 ? (f0 + warp) % 6 : f0 + fi;
       const bool owner = fi < F::FPI && f < 6;
       // the next faces (after the last: this CTA's next map's first) into L2 meanwhile
-      if (tid == 0 && (SS * 12) % 16 == 0) {
+      if (F::FPI > 1 && tid == 0 && (SS * 12) % 16 == 0) {
         const int n_pf = f0 + F::FPI >= 6 ? F::FPI : min(F::FPI, 6 - f0 - F::FPI);
         const long long nxt = f0 + F::FPI >= 6 ? (long long)(env + gridDim.x) * 6 : (long long)env * 6 + f0 + F::FPI;
         const float* pf = faces + (size_t)nxt * SS * 3;
