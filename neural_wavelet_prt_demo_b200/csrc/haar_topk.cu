@@ -78,6 +78,8 @@ constexpr int kScPrefix = 0, kScMask = 1, kScRemaining = 2, kScCounter = 3, kScE
 constexpr int kScListed = 14;                // cluster form: keys listed
 constexpr int kScNAbove = 16;                // batched kernel: keys in the final list
 constexpr int kScLevels = 17;                // batched kernel: winners written so far, those of level 2 apart: [2]
+constexpr int kScLeast = 19, kScMost = 20;   // batched kernel: of the keys marked
+constexpr int kScTied = 21;                  // batched kernel: the keys marked are all equal
 
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
@@ -700,20 +702,25 @@ __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
 // stored: the K winners' are recomputed from their texel blocks (block_coef).
 //
 // A map that overflows the first list goes over its keys once more; one whose last winner's bin is
-// too full (hundreds of equal keys) recomputes its keys in each pass of a radix select
-// (general_select).
+// crowded narrows it down, as a rule by the listed keys alone (settle_list).
 //
 // Small faces share the block: FPI of them are transformed at once.  Bound by L1 (69% busy) and issue
 // (63%): four CTAs of 64 registers fit an SM (107 us for 1,024 maps), and what they leave of the
 // SM's memory as L1 matters, since a texel row's three 16-byte loads share their sectors (lists of
 // 6 K + 768 keys instead of 5 K + 512 took one step of it: 110 -> 117 us).  1,024 maps, K = 300:
-// 132 us -> 107 (2,870 GB/s) with all keys kept in shared memory, three scans of them and two CTAs
-// per SM before; K = 64 109 -> 86, K = 1024 229 -> 202; S = 32 102 -> 50; S = 16, K = 64 67 -> 19;
-// maps of few lights on black 269 -> 84.  Of these, one prefix sum per list instead of a ballot per key and writing the
-// level-2 winners apart give 109.4 -> 107.1 (K = 64 86.4 -> 85.9, K = 1024 208.8 -> 202.3).
+// 134 us -> 106 (2,850 GB/s) with all keys kept in shared memory, three scans of them and two CTAs
+// per SM before; K = 64 112 -> 86, K = 1024 234 -> 212; S = 32 101 -> 47; S = 16, K = 64 70 -> 18;
+// black maps 298 -> 83; small whole numbers, K = 1024 311 -> 282 (radix select over the keys of the
+// map: 980).  Slower than with all keys kept: a plane gradient, whose level-2 details alone overflow
+// the list, 147 -> 169 (K = 64 102 -> 142).
 
 constexpr int kBins = 2048;       // of keys by bits 30..20
 constexpr int kCtasPerSm = 4;
+// Keys in the final list up to which the last winner's bin is not narrowed down: each is ranked among its
+// bin's.  1,024 maps of uniform noise, K = 300: 121 us, 129 from K + 192 keys on; K = 1024: 272, 305 from
+// K + K / 2 on.
+__host__ __device__ constexpr int uncrowded(int K) { return K + (K > 512 ? K / 4 : 128); }
+constexpr int kFineBins = 1024;   // settle_list: ten more bits; list_cap(1) composite keys hold them
 
 __host__ __device__ constexpr int map_coeffs(int S) { return 6 * S * S; }
 // Keys that may be listed while the faces pass, and in the end.
@@ -725,9 +732,10 @@ struct BatchSmem {
   uint32_t* hist;   // [kBins + 1] counts (from the second scan on: where the bin's next key goes); then 0
   uint32_t* lkey;   // [face_list_cap] keys listed while the faces pass
   uint16_t* lid;    // [face_list_cap] their coefficient: (face * NK + u) * kThreads + thread
-  uint32_t* bits;   // [6*S*S/32] aliases lkey: listed (zero fill) or tied (general_select) indices
-  uint32_t* wpre;   // [6*S*S/32] exclusive popcount prefix of bits (general_select)
+  uint32_t* bits;   // [6*S*S/32] in lkey's memory, after K of its entries: indices not to fill up with
+  uint32_t* wpre;   // [6*S*S/32] exclusive prefix of the zeros in bits
   uint64_t* gkey;   // [list_cap] composite keys of the final list
+  uint32_t* fine;   // [kFineBins] aliases gkey: counts of settle_list
   uint16_t* gid;    // [list_cap]
   uint16_t* order;  // [K] aliases lid: the winners' coefficients by rank
   uint16_t* turn;   // [K] aliases lkey: their ranks in the order they are written
@@ -742,8 +750,9 @@ __host__ __device__ inline size_t batch_smem_layout(int S, int K, char* base, Ba
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o = align16(o + bytes); return at; };
   const size_t oH = take(sizeof(uint32_t) * (kBins + 4));
-  const size_t list = align16(sizeof(uint32_t) * face_list_cap(S, K)), both = sizeof(uint32_t) * 2 * nw;
-  const size_t oL = take(list > both ? list : both);
+  const size_t list = align16(sizeof(uint32_t) * face_list_cap(S, K));
+  const size_t marks = sizeof(uint32_t) * 2 * nw, both = align16(sizeof(uint32_t) * K) + align16(marks);
+  const size_t oL = take(list > both ? list : both), oB = o - align16(marks);
   const size_t oI = take(sizeof(uint16_t) * face_list_cap(S, K));
   const size_t oG = take(sizeof(uint64_t) * list_cap(K));
   const size_t oD = take(sizeof(uint16_t) * list_cap(K));
@@ -757,8 +766,9 @@ __host__ __device__ inline size_t batch_smem_layout(int S, int K, char* base, Ba
     L->order = (uint16_t*)(base + oI);
     L->turn = (uint16_t*)(base + oL);
     L->lkey = (uint32_t*)(base + oL);
-    L->bits = (uint32_t*)(base + oL);
-    L->wpre = (uint32_t*)(base + oL) + nw;
+    L->bits = (uint32_t*)(base + oB);
+    L->wpre = (uint32_t*)(base + oB) + nw;
+    L->fine = (uint32_t*)(base + oG);
     L->lid = (uint16_t*)(base + oI);
     L->gkey = (uint64_t*)(base + oG);
     L->gid = (uint16_t*)(base + oD);
@@ -900,6 +910,44 @@ __device__ __forceinline__ uint32_t kth_bin_edge(const uint32_t* hist, int K, in
   return (uint32_t)(top - 2 * l2 - (in_b ? 1 : 0)) << 20;
 }
 
+// The fine bin that holds the n-th largest key counted so far (-1: fewer than n), by one warp.
+__device__ __forceinline__ int nth_fine_bin(const uint32_t* fine, int n, int lane) {
+  const volatile uint32_t* h = fine;
+  constexpr int PER = kFineBins / 32;
+  uint32_t sum = 0;
+#pragma unroll 8
+  for (int i = 0; i < PER; ++i) sum += h[kFineBins - PER * (lane + 1) + ((i + lane) & (PER - 1))];  // other banks
+  uint32_t incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  const uint32_t hit = __ballot_sync(0xffffffffu, incl >= (uint32_t)n);
+  if (!hit) return -1;
+  const int l = __ffs(hit) - 1, top = kFineBins - PER * l - 1;
+  const uint32_t before = __shfl_sync(0xffffffffu, incl - sum, l);
+  uint32_t in2 = h[top - lane];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, in2, o);
+    if (lane >= o) in2 += t;
+  }
+  const uint32_t hit2 = __ballot_sync(0xffffffffu, before + in2 >= (uint32_t)n);
+  return top - (hit2 ? __ffs(hit2) - 1 : 31);  // counts only grow: the bin is one of these 32
+}
+
+// Counts a warp's keys by bin, those of the first one's bin (often all: equal keys) with one atomic.
+__device__ __forceinline__ void count_key(uint32_t* counts, bool in, uint32_t bin, int lane) {
+  const uint32_t any = __ballot_sync(0xffffffffu, in);
+  if (!any) return;
+  const int lead = __ffs(any) - 1;
+  const uint32_t first = __shfl_sync(0xffffffffu, bin, lead);
+  const bool same = in && bin == first;
+  const uint32_t n = (uint32_t)__popc(__ballot_sync(0xffffffffu, same));
+  if (same ? lane == lead : in) atomicAdd(&counts[bin], same ? n : 1u);
+}
+
 // What a warp lists of the keys it forms (see above).
 struct KeyList {
   const BatchSmem& sm;
@@ -958,115 +1006,147 @@ struct KeyList {
   }
 };
 
-// Lists a map's keys once more, those from lo_key up (counts untouched).
-template <int S>
-__device__ __noinline__ void list_again(const float* map, uint32_t lo_key, int K) {
+// Goes over a map's keys once more.
+//  kList: lists those from lo up.
+//  kMark: lists those above [lo, lo + span), clears the bits of those in it and records the least and
+//         the largest of them.
+//  kNarrow: counts those in [lo, lo + span) by 1/1024 of it, and lists all from the running bound up
+//           that these counts give for the n-th largest of the interval.
+// Keys of 0 never take part.
+enum MapPass { kList, kMark, kNarrow };
+template <int S, MapPass PASS>
+__device__ __noinline__ void go_over_map(const float* map, int K, uint32_t lo, int span_bits, int n) {
   using F = FaceGeom<S>;
   extern __shared__ __align__(16) char smem_raw[];
   BatchSmem sm;
   batch_smem_layout(S, K, smem_raw, &sm);
-  const int tid = threadIdx.x, cap = face_list_cap(S, K);
-  KeyList list{sm, K, cap, tid & 31};
-  list.bound = lo_key;
+  static_assert(kFineBins / 32 == 32, "one bin a lane");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t first = max(lo, 1u), end = lo + (1u << span_bits);
+  KeyList list{sm, K, face_list_cap(S, K), lane};
+  list.bound = PASS == kMark ? end : first;
   const int lt = tid % F::T, fi = tid / F::T;
+  uint32_t least = ~0u, most = 0u;
   __syncthreads();
   if (tid == 0) sm.scal[kScListed] = 0;
+  if (PASS == kMark) {
+    for (int w = tid; w < (6 * F::SS + 31) / 32; w += kThreads) sm.bits[w] = ~0u;
+    if (tid == 0) sm.scal[kScLeast] = -1, sm.scal[kScMost] = 0;
+  }
+  if (PASS == kNarrow)
+    for (int i = tid; i < kFineBins; i += kThreads) sm.fine[i] = 0u;
   __syncthreads();
 #pragma unroll 1
   for (int f0 = 0; f0 < 6; f0 += F::FPI) {
-    const int f = f0 + fi;
+    const int f = F::FPI == 1 ? (f0 + warp) % 6 : f0 + fi;  // kNarrow: the first counts see all faces
     const bool owner = fi < F::FPI && f < 6;
     uint32_t k[F::NK];
     float ll[3];
     face_keys<S>(map + (size_t)f * F::SS * 3, owner, lt, k, ll);
     const float* upf = sm.up + f * 3 * kThreads;
     if (owner) k[F::NR] = wavelet_key_bits(upf[lt], upf[kThreads + lt], upf[2 * kThreads + lt]);
+    if constexpr (PASS == kNarrow) {
+#pragma unroll
+      for (int u = 0; u < F::NK; ++u)
+        count_key(sm.fine, k[u] >= list.bound && k[u] < end, (k[u] - lo) >> (span_bits - 10), lane);
+      if (f0 == 0) __syncthreads();  // without the first counts no bound
+      const int b = nth_fine_bin(sm.fine, n, lane);
+      if (b >= 0) list.bound = max(list.bound, lo + ((uint32_t)b << (span_bits - 10)));
+    }
     list.add(k, F::NK, true, [&](int u) { return (f * F::NK + u) * kThreads + lt; });
+    if constexpr (PASS == kMark) {
+#pragma unroll
+      for (int u = 0; u < F::NK; ++u)
+        if (k[u] >= first && k[u] < end) {
+          const int g = f * F::SS + flat_in_face<S>(lt, u);
+          atomicAnd(&sm.bits[g >> 5], ~(1u << (g & 31)));
+          least = min(least, k[u]);
+          most = max(most, k[u]);
+        }
+    }
+  }
+  if constexpr (PASS == kMark) {
+    least = __reduce_min_sync(0xffffffffu, least);
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0) {
+      atomicMin(reinterpret_cast<uint32_t*>(&sm.scal[kScLeast]), least);
+      atomicMax(reinterpret_cast<uint32_t*>(&sm.scal[kScMost]), most);
+    }
   }
   __syncthreads();
 }
 
-// The K winners of a map whose lists overflowed, into gkey / gid: a 4-pass 8-bit radix select that
-// recomputes the keys in each pass, then ties at the threshold in flat-index order by a bitmap.
+// Completes the list where the faces' pass left it incomplete or the last winner's bin crowded.
+//
+// A list that overflowed is made again from that bin up.  A crowded bin is narrowed down, ten bits at a time, by the listed keys or, where the list overflowed, by
+// going over the map again.  This ends with the keys from a fine bin's lower edge up listed or, if a fine
+// bin holds too many equal ones, with those above it listed and its own marked: they are taken in
+// flat-index order.  Leaves the lower edge of the listed keys, their number and whether equal ones are
+// marked in scal.
 template <int S>
-__device__ __noinline__ void general_select(const float* map, int K) {
-  using F = FaceGeom<S>;
+__device__ __noinline__ void settle_list(const float* map, int K) {
   extern __shared__ __align__(16) char smem_raw[];
   BatchSmem sm;
   batch_smem_layout(S, K, smem_raw, &sm);
-  const float* up = sm.up;
-  constexpr int SS = F::SS, NR = F::NR, NK = F::NK, NW = (6 * SS + 31) / 32;
-  const int tid = threadIdx.x, lt = tid % F::T, fi = tid / F::T;
-  uint32_t prefix = 0, mask = 0, thr = 0;
-  int remaining = K, n_sel = 0, slot = 0;
-  __syncthreads();
-  for (int w = tid; w < NW; w += kThreads) sm.bits[w] = 0u;
-  // passes 0-3: the threshold; 4: the ties' bitmap; 5: each thread's winners; 6: their slots
-  for (int pass = 0; pass < 7; ++pass) {
-    const int shift = 24 - 8 * pass;
-    if (pass < 4) sm.hist[tid] = 0u;
-    __syncthreads();
-    if (pass == 5) {
-      constexpr int PER = (NW + kThreads - 1) / kThreads;
-      uint32_t mine = 0, all;
-      for (int i = 0; i < PER; ++i) mine += tid * PER + i < NW ? (uint32_t)__popc(sm.bits[tid * PER + i]) : 0u;
-      uint32_t run = block_inclusive_sum(mine, sm.warp_tot, &all) - mine;
-      for (int i = 0; i < PER; ++i)
-        if (tid * PER + i < NW) {
-          sm.wpre[tid * PER + i] = run;
-          run += (uint32_t)__popc(sm.bits[tid * PER + i]);
-        }
-      __syncthreads();
-    }
-    if (pass == 6) {
-      uint32_t all;
-      slot = (int)block_inclusive_sum((uint32_t)n_sel, sm.warp_tot, &all) - n_sel;
-    }
-    for (int f = fi; f < 6 && fi < F::FPI; f += F::FPI) {
-      uint32_t k[NK];
-      float ll[3];
-      face_keys<S>(map + (size_t)f * SS * 3, true, lt, k, ll);
-      const float* upf = up + f * 3 * kThreads;
-      k[NR] = wavelet_key_bits(upf[lt], upf[kThreads + lt], upf[2 * kThreads + lt]);
-#pragma unroll
-      for (int u = 0; u < NK; ++u) {
-        if (pass < 4) {
-          if ((k[u] & mask) == prefix) atomicAdd(&sm.hist[(k[u] >> shift) & 255u], 1u);
-          continue;
-        }
-        if (k[u] < thr) continue;
-        const int g = f * SS + flat_in_face<S>(lt, u), w = g >> 5;
-        if (pass == 4) {
-          if (k[u] == thr) atomicOr(&sm.bits[w], 1u << (g & 31));
-          continue;
-        }
-        if (k[u] == thr && (int)(sm.wpre[w] + __popc(sm.bits[w] & ((1u << (g & 31)) - 1u))) >= remaining) continue;
-        if (pass == 5) {
-          ++n_sel;
-        } else {
-          sm.gkey[slot] = ((uint64_t)k[u] << 32) | (uint64_t)(0xFFFFFFFFu - (uint32_t)g);
-          sm.gid[slot] = (uint16_t)((f * NK + u) * kThreads + lt);
-          ++slot;
-        }
-      }
-    }
-    __syncthreads();
-    if (pass < 4) {
-      const int digit = 255 - tid;
-      uint32_t all;
-      const uint32_t tot = sm.hist[digit];
-      const uint32_t incl = block_inclusive_sum(tot, sm.warp_tot, &all);
-      if (incl >= (uint32_t)remaining && incl - tot < (uint32_t)remaining) {
-        sm.scal[kScPrefix] = (int)(prefix | ((uint32_t)digit << shift));
-        sm.scal[kScRemaining] = remaining - (int)(incl - tot);
-      }
-      __syncthreads();
-      prefix = (uint32_t)sm.scal[kScPrefix];
-      remaining = sm.scal[kScRemaining];
-      mask |= 255u << shift;
-      thr = prefix;
-    }
+  const int tid = threadIdx.x, lane = tid & 31, cap = face_list_cap(S, K);
+  uint32_t lo = (uint32_t)sm.scal[kScPrefix];
+  if (sm.scal[kScNAbove] <= uncrowded(K)) {
+    go_over_map<S, kList>(map, K, lo, 0, 0);
+    return;
   }
+  int n_above = (int)sm.hist[lo >> 20];  // where the bin's part of the final list starts
+  lo = lo >> 20 << 20;
+  bool listed = sm.scal[kScListed] <= cap;  // every key from the bin up is
+  for (int bits = 20; bits > 0; bits -= 10) {
+    if (listed) {
+      const int n_all = sm.scal[kScListed];
+      __syncthreads();
+      for (int i = tid; i < kFineBins; i += kThreads) sm.fine[i] = 0u;
+      __syncthreads();
+      for (int e0 = tid - lane; e0 < n_all; e0 += kThreads) {
+        const uint32_t k = e0 + lane < n_all ? sm.lkey[e0 + lane] : 0u;
+        count_key(sm.fine, k >= max(lo, 1u) && k < lo + (1u << bits), (k - lo) >> (bits - 10), lane);
+      }
+      __syncthreads();
+    } else {
+      go_over_map<S, kNarrow>(map, K, lo, bits, K - n_above);
+      listed = sm.scal[kScListed] <= cap;
+    }
+    const int b0 = kFineBins - 4 - 4 * tid;
+    const uint4 v = *reinterpret_cast<const uint4*>(sm.fine + b0);
+    const uint32_t c[4] = {v.x, v.y, v.z, v.w}, sum = v.x + v.y + v.z + v.w;
+    uint32_t all;
+    uint32_t run = (uint32_t)n_above + block_inclusive_sum(sum, sm.warp_tot, &all) - sum;
+#pragma unroll
+    for (int i = 3; i >= 0; --i) {
+      if (run < (uint32_t)K && run + c[i] >= (uint32_t)K) {
+        sm.scal[kScPrefix] = b0 + i;
+        sm.scal[kScNAbove] = (int)run;
+        sm.scal[kScRemaining] = (int)c[i];
+      }
+      run += c[i];
+    }
+    __syncthreads();
+    lo += (uint32_t)sm.scal[kScPrefix] << (bits - 10);
+    n_above = sm.scal[kScNAbove];
+    const int n = sm.scal[kScRemaining];
+    __syncthreads();
+    const bool fits = n_above + n <= list_cap(K);
+    if (n_above + n <= uncrowded(K) || (bits == 10 && fits)) {
+      if (!listed) go_over_map<S, kList>(map, K, lo, 0, 0);
+      if (tid == 0) sm.scal[kScPrefix] = (int)max(lo, 1u), sm.scal[kScNAbove] = n_above + n;
+      break;
+    }
+    if (bits == 20 && (listed || fits)) continue;
+    go_over_map<S, kMark>(map, K, lo, bits - 10, 0);
+    if (bits == 10 || sm.scal[kScLeast] == sm.scal[kScMost]) {
+      if (tid == 0)
+        sm.scal[kScPrefix] = (int)(lo + (1u << (bits - 10))), sm.scal[kScNAbove] = n_above, sm.scal[kScTied] = 1;
+      break;
+    }
+    listed = false;  // the list holds those above only
+  }
+  __syncthreads();
 }
 
 template <int S>
@@ -1179,7 +1259,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     if (tid == 0) {
       sm.scal[kScPrefix] = 1;  // every listed key, if they are fewer than K
       sm.scal[kScNAbove] = -1;
-      sm.scal[kScLevels] = sm.scal[kScLevels + 1] = 0;
+      sm.scal[kScLevels] = sm.scal[kScLevels + 1] = sm.scal[kScTied] = 0;
     }
     __syncthreads();
     // ---- the last winner's bin: eight bins a thread from the top.  A bin's part of the final list
@@ -1209,29 +1289,19 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       if (tid == kThreads - 1 && all < (uint32_t)K) sm.scal[kScNAbove] = (int)all;
     }
     __syncthreads();
+    if (__builtin_expect(sm.scal[kScNAbove] > uncrowded(K) || *n_listed > cap, 0)) settle_list<S>(map, K);
     const uint32_t lo_key = (uint32_t)sm.scal[kScPrefix];
-    int n_all = *n_listed, n_final = sm.scal[kScNAbove];
-    if (n_all > cap && n_final <= list_cap(K)) {
-      // the list overflowed (faces each brighter than the one before), but the counts are whole
-      list_again<S>(map, lo_key, K);
-      n_all = *n_listed;
+    const int n_all = *n_listed, n_final = sm.scal[kScNAbove];
+    for (int e = tid; e < n_all; e += kThreads) {
+      const uint32_t k = sm.lkey[e];
+      if (k < lo_key) continue;
+      const int id = sm.lid[e], t = id % kThreads, fu = id / kThreads, f = fu / NK, u = fu % NK;
+      const int g = f * SS + flat_in_face<S>(t, u);
+      const uint32_t slot = atomicAdd(&sm.hist[k >> 20], 1u);
+      sm.gkey[slot] = ((uint64_t)k << 32) | (uint64_t)(0xFFFFFFFFu - (uint32_t)g);
+      sm.gid[slot] = (uint16_t)id;
     }
-    const bool general = n_all > cap || n_final > list_cap(K);
-    if (!general) {
-      for (int e = tid; e < n_all; e += kThreads) {
-        const uint32_t k = sm.lkey[e];
-        if (k < lo_key) continue;
-        const int id = sm.lid[e], t = id % kThreads, fu = id / kThreads, f = fu / NK, u = fu % NK;
-        const int g = f * SS + flat_in_face<S>(t, u);
-        const uint32_t slot = atomicAdd(&sm.hist[k >> 20], 1u);
-        sm.gkey[slot] = ((uint64_t)k << 32) | (uint64_t)(0xFFFFFFFFu - (uint32_t)g);
-        sm.gid[slot] = (uint16_t)id;
-      }
-      __syncthreads();
-    } else {
-      general_select<S>(map, K);
-      n_final = K;
-    }
+    __syncthreads();
     // one channel of a winner: its strength (and, with the first, its index)
     auto put = [&](int rank, int c, int id) {
       const int t = id % kThreads, fu = id / kThreads, f = fu / NK, u = fu % NK;
@@ -1246,23 +1316,26 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       const uint64_t me = sm.gkey[e];
       // its bin's part ends where the bin's next key would go, and starts where the bin above ends
       const uint32_t bin = (uint32_t)(me >> 52);
-      int rank = general ? 0 : (int)sm.hist[bin + 1];
+      int rank = (int)sm.hist[bin + 1];
       const uint64_t* o = sm.gkey + rank;
-      const int n = (general ? K : (int)sm.hist[bin]) - rank;
+      const int n = (int)sm.hist[bin] - rank;
 #pragma unroll 4
       for (int i = 0; i < n; ++i) rank += o[i] > me;
       if (rank < K) sm.order[rank] = sm.gid[e];
     }
     if (n_final < K) {
-      // ---- fewer than K keys above 0: then the coefficients not listed, in flat-index order
+      // ---- then equal keys in flat-index order: those marked or, if fewer than K keys are above 0, the
+      // coefficients not listed
       constexpr int NW = (6 * SS + 31) / 32, PER = (NW + kThreads - 1) / kThreads;
-      for (int w = tid; w < NW; w += kThreads) sm.bits[w] = w * 32 + 32 <= 6 * SS ? 0u : ~0u << (6 * SS - w * 32);
-      __syncthreads();
-      for (int e = tid; e < n_final; e += kThreads) {
-        const uint32_t g = 0xFFFFFFFFu - (uint32_t)sm.gkey[e];
-        atomicOr(&sm.bits[g >> 5], 1u << (g & 31));
+      if (!sm.scal[kScTied]) {
+        for (int w = tid; w < NW; w += kThreads) sm.bits[w] = w * 32 + 32 <= 6 * SS ? 0u : ~0u << (6 * SS - w * 32);
+        __syncthreads();
+        for (int e = tid; e < n_final; e += kThreads) {
+          const uint32_t g = 0xFFFFFFFFu - (uint32_t)sm.gkey[e];
+          atomicOr(&sm.bits[g >> 5], 1u << (g & 31));
+        }
+        __syncthreads();
       }
-      __syncthreads();
       uint32_t mine = 0, all;
       for (int i = 0; i < PER; ++i) mine += tid * PER + i < NW ? 32u - (uint32_t)__popc(sm.bits[tid * PER + i]) : 0u;
       uint32_t run = block_inclusive_sum(mine, sm.warp_tot, &all) - mine;

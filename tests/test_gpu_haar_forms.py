@@ -91,3 +91,62 @@ def test_ever_brighter_faces_are_not_read_twice(cuda):
     maps = torch.exp(1.5 * torch.randn((1024, 6, 64, 64, 3), generator=g, device=cuda))
     brighter = maps * (10.0 ** torch.arange(6.0, device=cuda)).view(1, 6, 1, 1, 1)
     assert _median_us(brighter, 300) < 1.3 * _median_us(maps, 300)
+
+
+# Maps whose last winner shares its bin with hundreds of others, which the batched form narrows down or
+# takes in flat-index order, and maps whose faces grow brighter.
+def _crowded(S, kind, seed):
+    g = np.random.default_rng(seed)
+    ramp = np.add.outer(np.linspace(0, 1, S), np.linspace(0, 2, S))[None, :, :, None] * np.ones((6, 1, 1, 3))
+    quad = np.kron(np.ones((S // 2, S // 2)), [[1.0, -1.0], [1.0, -1.0]])[None, :, :, None] * np.ones((6, 1, 1, 3))
+    if kind == "ramp":                                                   # hundreds of nearly equal slopes
+        return ramp + 1e-3 * g.random((6, S, S, 3))
+    if kind == "equal slopes":                                           # equal up to rounding
+        return ramp
+    if kind == "ints":                                                   # few values, many of each
+        return g.integers(0, 3, (6, S, S, 3))
+    if kind == "lights on equals":                                       # a few above hundreds of equal ones
+        return quad + 100.0 * (g.random((6, S, S, 1)) < 2e-3)
+    if kind == "last bits":                                              # equal but for the last ten bits
+        return quad * (1 + g.integers(0, 900, (6, S // 2, S // 2, 1)).repeat(2, 1).repeat(2, 2) * 2.0 ** -23)
+    if kind == "last bits and equals":                                   # of these, one value hundreds of times
+        u = g.integers(0, 900, (6, S // 2, S // 2, 1)) * (g.random((6, S // 2, S // 2, 1)) < 0.1)
+        return quad * (1 + u.repeat(2, 1).repeat(2, 2) * 2.0 ** -23)
+    if kind == "equal subnormals":
+        return quad * 3e-40
+    if kind == "subnormals":
+        return quad * 1e-40 * g.integers(1, 900, (6, S // 2, S // 2, 1)).repeat(2, 1).repeat(2, 2)
+    if kind == "ever brighter":
+        return np.exp(1.5 * g.standard_normal((6, S, S, 3))) * 10.0 ** np.arange(6).reshape(6, 1, 1, 1)
+    return ramp * 10.0 ** -np.arange(6).reshape(6, 1, 1, 1)              # ever darker ramps
+
+
+KINDS = ["ramp", "equal slopes", "ints", "lights on equals", "last bits", "last bits and equals", "equal subnormals",
+         "subnormals", "ever brighter", "ever darker ramps"]
+
+
+@pytest.mark.parametrize("S,K", [(64, 300), (64, 1), (64, 64), (64, 1024), (32, 300), (32, 1024), (16, 40), (16, 1024),
+                                 (8, 384)])
+def test_crowded_bins_bit_exact(cuda, S, K):
+    # more maps than CTAs, so that each kind is followed by another on the same CTA
+    import torch
+    from neural_wavelet_prt_demo_b200 import engine as eng
+    E = 8 * torch.cuda.get_device_properties(0).multi_processor_count
+    base = np.stack([_crowded(S, k, i) for i, k in enumerate(KINDS)]).astype(np.float32)
+    pick = np.random.default_rng(S + K).integers(0, len(KINDS), E)
+    idx, st = eng.haar_topk(torch.from_numpy(base).to(cuda)[torch.from_numpy(pick).to(cuda)].contiguous(), K)
+    ridx, rst = O.haar_topk(base, K)
+    bad = np.nonzero((idx.cpu().numpy() != ridx[pick]).any(axis=1))[0]
+    assert bad.size == 0, sorted({KINDS[pick[b]] for b in bad})
+    assert bits_equal(st.cpu().numpy(), rst[pick])
+    one = [eng.haar_topk(torch.from_numpy(m).to(cuda), K) for m in base]  # the cluster form
+    assert all(np.array_equal(i.cpu().numpy(), r) for (i, _), r in zip(one, ridx))
+
+
+def test_equal_keys_do_not_take_pass_after_pass(cuda):
+    # 4.8 times as long as ordinary maps when a radix select went over the map for each digit
+    import torch
+    g = torch.Generator(device=cuda).manual_seed(5)
+    maps = torch.exp(1.5 * torch.randn((1024, 6, 64, 64, 3), generator=g, device=cuda))
+    ints = torch.randint(0, 3, maps.shape, generator=g, device=cuda).float()
+    assert _median_us(ints, 1024) < 2.0 * _median_us(maps, 1024)
