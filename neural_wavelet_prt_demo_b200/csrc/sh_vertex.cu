@@ -18,7 +18,10 @@
 //    bulk copy, a head and a tail of at most three floats by cp.async.
 //  * n a multiple of 4, T 16-byte aligned: rows an odd number of 16-byte chunks apart, read four
 //    terms at a time.  One bulk copy where n / 4 is odd, else one per row.
-//  * otherwise: an odd stride, by 4-byte cp.async.
+//  * other even n, up to 8-way conflicts: as in memory all the same.  60 MB of matrices of 62: 18.5 us, 51.4 by 4-byte copies to an odd stride; of 72 (8-way) with T on no 16-byte
+//    boundary 27.0 and 45.8.
+//  * otherwise (multiples of 16 with T on no 16-byte boundary, and n = 2, 51.4 us against 55.4): an
+//    odd stride, by 4-byte cp.async.  Matrices of 48: 37.8 us, of 80: 35.0.
 // 40,000 vertices of 81 coefficients: 249 us with one row at a time (three env SH reads per term
 // and row) and 16-byte cp.async, 201 with three rows side by side, 157 with bulk copies (6,930
 // GB/s); 14,364 of 64: 277 us (32-way conflicts), 148 by 4-byte copies to an odd stride, 67 by
@@ -33,14 +36,14 @@ namespace {
 constexpr int kMaxN = 81;
 constexpr int kWarps = 8;
 
-enum RowForm { kOddRows, kChunkRows, kSingles };  // how a matrix is staged (above)
+enum RowForm { kOddRows, kChunkRows, kEvenRows, kSingles };  // how a matrix is staged (above)
 
 // Shared memory in floats: the env SH (padded to 4 per coefficient), then per warp light[k] and
 // brdf[v] ([kMaxN][3] each), then per warp a T staging area plus up to 3 of alignment shift,
 // rounded to 16 bytes.
 __host__ __device__ constexpr int stage_offset() { return (4 * kMaxN + 2 * kWarps * kMaxN * 3 + 3) & ~3; }
 __host__ __device__ constexpr int row_stride(int n, RowForm form) {
-  return form == kChunkRows ? ((n / 4) | 1) * 4 : n | 1;
+  return form == kChunkRows ? ((n / 4) | 1) * 4 : form == kEvenRows ? n : n | 1;
 }
 __host__ __device__ constexpr int stage_stride(int n, RowForm form) { return (n * row_stride(n, form) + 3 + 3) & ~3; }
 
@@ -73,7 +76,7 @@ __global__ void __launch_bounds__(kWarps * 32) sh_vertex_kernel(const float* __r
     const float* src = T + v * nn;
     const float* bsrc = brdf + v * n * 3;
     float* t = stage;
-    if constexpr (FORM == kOddRows) {
+    if constexpr (FORM == kOddRows || FORM == kEvenRows) {
       // t[i] and src[i] share their offset modulo 16 bytes
       const int mis = (int)((reinterpret_cast<uintptr_t>(src) >> 2) & 3);
       t += mis;
@@ -230,9 +233,11 @@ void launch_sh_vertex(const float* T, const float* brdf, const float* L, int64_t
     else if (n <= 64) go(sh_vertex_kernel<2, F>, F);
     else go(sh_vertex_kernel<3, F>, F);
   };
-  // every row of a T[v] starts on a 16-byte boundary if T does and n is a multiple of 4
+  // every row of a T[v] starts on a 16-byte boundary if T does and n is a multiple of 4 (odd and even
+  // rows: one form each, as an odd stride known to the compiler takes n = 81 from 16.5 to 14.5 us)
   if (n % 2) rows(std::integral_constant<RowForm, kOddRows>{});
   else if (n % 4 == 0 && (reinterpret_cast<uintptr_t>(T) & 15) == 0) rows(std::integral_constant<RowForm, kChunkRows>{});
+  else if (n % 16 && n > 2) rows(std::integral_constant<RowForm, kEvenRows>{});
   else rows(std::integral_constant<RowForm, kSingles>{});
   NWPRT_CUDA(cudaGetLastError());
 }
