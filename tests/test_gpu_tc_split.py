@@ -110,3 +110,87 @@ def test_infinite_last_term_gives_infinity(cuda, w, h, K):
     assert not np.isnan(out[0]).any()
     assert np.isinf(out[0]).any() and np.array_equal(np.isinf(out[0]), np.isinf(out[1]))
     e.close()
+
+
+def _pixels(sms, rounds, rest):
+    """Pixels of `rounds` whole rounds of tiles (five a CTA) and `rest` more tiles, the last one ragged."""
+    return (rounds * 5 * sms + rest) * 128 - 37
+
+
+def _part(gb, begin, end):
+    import dataclasses
+    return dataclasses.replace(gb, width=end - begin, height=1, **{
+        f: getattr(gb, f)[begin:end] for f in ("pos", "normal", "reflect", "roughness", "kd", "ks", "direct", "flag")})
+
+
+@pytest.mark.parametrize("cfg,precision,rounds,rest,K", [
+    ("small", "bf16", 2, 1, 6),     # tiles from the counter, then one shared
+    ("small", "bf16", 2, 290, 13),  # then two per SM
+    ("small", "bf16", 3, 300, 6),   # first encodings staggered, counter, a partial round of whole tiles (small K)
+    ("large", "bf16", 3, 290, 13),  # staggered, counter, shared
+    ("large", "bf16", 21, 660, 13),  # a 1080p frame: staggered, counter, nothing shared
+    ("large", "fp8", 3, 140, 6),
+])
+def test_launches_of_several_rounds(cuda, cfg, precision, rounds, rest, K):
+    import torch
+    from neural_wavelet_prt_demo_b200 import engine as eng, synth
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    case = make_case(netconfig.CONFIG_SMALL if cfg == "small" else netconfig.CONFIG_LARGE, 64, 4, K, seed=K,
+                     hash_scale=0.5)
+    n = _pixels(sms, rounds, rest)
+    gb = synth.make_gbuffer(n, 1, seed=rounds, flag_prob=0.9)
+    e = eng.RenderEngine(case.cfg)
+    e.loadWeights(case.weights)
+    env = e.addEnvironmentMap(eng.EnvironmentMap(top_coefficients=case.idx, top_strength=case.strength))
+    fr = eng.FullFrame.from_gbuffer(gb)
+    e.setFrame(0, fr)
+    e.TCNNPass_p1(0)
+    if precision == "fp8":
+        e.calibrateFP8(env, 0, 0, 4096)
+    rc = eng.RenderConfig(precision=precision)
+    fr.fbPredictedIndirect.fill_(float("nan"))
+    e.TCNNPass_p2(env, 0, rc)
+    e.TCNNSync()
+    whole = fr.fbPredictedIndirect.clone(), fr.fbPredictedIndirectWithDirect.clone()
+    # alone: pieces of at most a round, whose tiles are a warpgroup's or shared
+    for t in (fr.fbPredictedIndirect, fr.fbPredictedIndirectWithDirect):
+        t.fill_(float("nan"))
+    for b in range(0, n, 700 * 128):
+        e.relightRanges([(env, 0, fr.fbPredictedIndirect, fr.fbPredictedIndirectWithDirect, b, min(n, b + 700 * 128))], rc)
+    e.TCNNSync()
+    for got, ref in zip(whole, (fr.fbPredictedIndirect, fr.fbPredictedIndirectWithDirect)):
+        assert torch.equal(got.view(torch.int32), ref.view(torch.int32))
+    # pixels of the first, a later and the last tiles against 64 bits
+    for b in (0, n // 2, n - 500):
+        part = _part(gb, b, b + 500)
+        r64 = O.relight_f64(O.Bound(case.desc, case.weights, part), case.idx, case.strength)
+        assert psnr(whole[0][b:b + 500, :3].cpu().numpy(), r64) >= (30.0 if precision == "fp8" else PSNR_MIN)
+    e.close()
+
+
+def test_jobs_of_different_wavelet_counts_in_several_rounds(cuda):
+    # tiles of different cost: all from the counter, none shared
+    import torch
+    from neural_wavelet_prt_demo_b200 import engine as eng, synth
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    cases = [make_case(netconfig.CONFIG_SMALL, 64, 4, K, seed=3, hash_scale=0.5) for K in (6, 40)]
+    e = eng.RenderEngine(cases[0].cfg)
+    e.loadWeights(cases[0].weights)
+    rc = eng.RenderConfig(precision="bf16")
+    jobs, frames = [], []
+    for i, (case, tiles) in enumerate(zip(cases, (6 * sms, 5 * sms + 11))):
+        env = e.addEnvironmentMap(eng.EnvironmentMap(top_coefficients=case.idx, top_strength=case.strength))
+        fr = eng.FullFrame.from_gbuffer(synth.make_gbuffer(tiles * 128 - 19, 1, seed=i, flag_prob=0.9))
+        e.setFrame(i, fr)
+        e.TCNNPass_p1(i)
+        frames.append(fr)
+        jobs.append((env, i, fr.fbPredictedIndirect, fr.fbPredictedIndirectWithDirect, 0, 0))
+    e.relightRanges(jobs, rc)
+    e.TCNNSync()
+    together = [fr.fbPredictedIndirect.clone() for fr in frames]
+    for job in jobs:
+        e.relightRanges([job], rc)
+    e.TCNNSync()
+    for fr, t in zip(frames, together):
+        assert torch.equal(t.view(torch.int32), fr.fbPredictedIndirect.view(torch.int32))
+    e.close()
