@@ -35,10 +35,11 @@ inline void cuda_check(cudaError_t e, const char* what) {
 // (programmatic dependent launch; behind anything but a kernel it is an ordinary launch).  Such a
 // kernel calls stream_wait before its first access to memory that earlier work in the stream may
 // use, so what it does before that must touch only shared and tensor memory, its parameters and
-// weights (which only host-synchronous copies write).  A short call's time is half launch latency
-// and prologue: G-buffer pass + tensor-core relight at 128 x 128 30.8 -> 26.6 us, SH projection at
-// S = 128 14.3 -> 11.5, tonemap at 2559 x 1439 15.1 -> 13.7, rotate + wavelets 19.2 -> 18.3, a
-// serving request with a rotated map 218 -> 212.  The per-vertex SH pass and the FP32 relight got no
+// weights (which only host-synchronous copies write), and it reads what that work may write by
+// ld_stream.  A short call's time is half launch latency and prologue: G-buffer pass + tensor-core
+// relight at 128 x 128 30.7 -> 26.5 us, SH projection at S = 128 14.3 -> 11.8, tonemap at 2559 x 1439
+// 15.7 -> 14.2, rotate + wavelets 19.5 -> 18.9, a serving request with a rotated map 218.6 -> 214.3
+// (calls in a loop, with overlap off and on).  The per-vertex SH pass and the FP32 relight got no
 // faster by it (185 -> 197 us, 16.65 -> 16.67 ms) and are launched as usual.
 template <class... P, class... A>
 inline void launch_overlapped(void (*kern)(P...), long long grid, int block, size_t smem, cudaStream_t st, A&&... args) {

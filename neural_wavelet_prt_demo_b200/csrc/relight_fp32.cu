@@ -18,8 +18,8 @@
 // costs 17 loads for the same 32 (the weights are not reused): shared-memory reads bounded it.
 // The warp's rows are its own, so layers need no block barrier.  The rows of a layer are unrolled
 // by 32, the period of the swizzle, which leaves no address arithmetic in the loop.
-// 1080p network, 611 x 407, K = 64: 28.2 -> 16.7 ms (59% of the FP32 pipe's peak; 55.7 kFLOP per
-// evaluation); 128 x 128 network, 128 x 128, K = 64: 610 -> 453 us.
+// 1080p network, 611 x 407, K = 64: 28.2 -> 16.7 ms (51.3 TFLOP/s of the reference network's 53.6 kFLOP per
+// evaluation, 69% of the FP32 pipe's nominal 74); 128 x 128 network, 128 x 128, K = 64: 610 -> 453 us.
 #include <cmath>
 
 #include "nwprt_internal.cuh"
