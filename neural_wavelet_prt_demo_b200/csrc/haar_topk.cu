@@ -689,9 +689,8 @@ __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
 // what came before), and from step to step once the list is crowded.  A step of a 64 x 64 map is an
 // eighth of a face per warp, of another face each, so that the first one sees all of them: face by
 // face, maps whose faces grow brighter listed too much and were read twice (each ten times brighter
-// than the one before: 173 us, now 95; twice: 132, now 101).  No single copy can fetch the next step
-// ahead then, which four CTAs per SM do without (line by line: 110.7 against 107.2 us; three per SM,
-// K = 1024: 203 -> 212).  Taking the faces by a sample of their detail, the largest first: 112.2 us.
+// than the one before: 173 us, now 93; twice: 132, now 99).  No single copy can fetch the next step
+// ahead then, which the CTAs of an SM do without (line by line: 110.7 against 107.2 us).  Taking the faces by a sample of their detail, the largest first: 112.2 us.
 // No barrier guards the look-up: counts still missing only lower the bound.  When the upper levels
 // are done, one block scan over the bins gives the last winner's bin, the listed keys from it up go
 // to their bin's part of a second list, and each is ranked among its own bin's keys only.  Keys
@@ -708,17 +707,17 @@ __global__ void __cluster_dims__(6, 1, 1) __launch_bounds__(kThreads, 2)
 // (63%): four CTAs of 64 registers fit an SM (107 us for 1,024 maps), and what they leave of the
 // SM's memory as L1 matters, since a texel row's three 16-byte loads share their sectors (lists of
 // 6 K + 768 keys instead of 5 K + 512 took one step of it: 110 -> 117 us).  1,024 maps, K = 300:
-// 134 us -> 106 (2,850 GB/s) with all keys kept in shared memory, three scans of them and two CTAs
-// per SM before; K = 64 112 -> 86, K = 1024 234 -> 212; S = 32 101 -> 47; S = 16, K = 64 70 -> 18;
-// black maps 298 -> 83; small whole numbers, K = 1024 311 -> 282 (radix select over the keys of the
+// 134 us -> 104 (2,950 GB/s) with all keys kept in shared memory, three scans of them and two CTAs
+// per SM before; K = 64 112 -> 84, K = 1024 234 -> 200; S = 32 101 -> 46; S = 16, K = 64 70 -> 18;
+// black maps 298 -> 79; small whole numbers, K = 1024 311 -> 265 (radix select over the keys of the
 // map: 980).  Slower than with all keys kept: a plane gradient, whose level-2 details alone overflow
-// the list, 147 -> 169 (K = 64 102 -> 142).
+// the list, 147 -> 168 (K = 64 102 -> 136).
 
 constexpr int kBins = 2048;       // of keys by bits 30..20
 constexpr int kCtasPerSm = 4;
 // Keys in the final list up to which the last winner's bin is not narrowed down: each is ranked among its
 // bin's.  1,024 maps of uniform noise, K = 300: 121 us, 129 from K + 192 keys on; K = 1024: 272, 305 from
-// K + K / 2 on.
+// K + K / 2 on (with settle_list a call).
 __host__ __device__ constexpr int uncrowded(int K) { return K + (K > 512 ? K / 4 : 128); }
 constexpr int kFineBins = 1024;   // settle_list: ten more bits; list_cap(1) composite keys hold them
 
@@ -1015,7 +1014,7 @@ struct KeyList {
 // Keys of 0 never take part.
 enum MapPass { kList, kMark, kNarrow };
 template <int S, MapPass PASS>
-__device__ __noinline__ void go_over_map(const float* map, int K, uint32_t lo, int span_bits, int n) {
+__device__ __forceinline__ void go_over_map(const float* map, int K, uint32_t lo, int span_bits, int n) {
   using F = FaceGeom<S>;
   extern __shared__ __align__(16) char smem_raw[];
   BatchSmem sm;
@@ -1082,9 +1081,10 @@ __device__ __noinline__ void go_over_map(const float* map, int K, uint32_t lo, i
 // going over the map again.  This ends with the keys from a fine bin's lower edge up listed or, if a fine
 // bin holds too many equal ones, with those above it listed and its own marked: they are taken in
 // flat-index order.  Leaves the lower edge of the listed keys, their number and whether equal ones are
-// marked in scal.
+// marked in scal.  Inlined, rare as it is: around a call the kernel's 64 registers spill in every step
+// (K = 64, 300 and 1024: 86.3, 106.2 and 210.5 us with a call, 83.7, 104.0 and 199.7 without).
 template <int S>
-__device__ __noinline__ void settle_list(const float* map, int K) {
+__device__ __forceinline__ void settle_list(const float* map, int K) {
   extern __shared__ __align__(16) char smem_raw[];
   BatchSmem sm;
   batch_smem_layout(S, K, smem_raw, &sm);
